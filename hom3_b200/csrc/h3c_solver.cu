@@ -31,6 +31,7 @@
 #include "muscl_adjoint.cuh"
 #include "cns_adjoint.cuh"
 #include "stage_halo.hpp"
+#include "stage_split.hpp"
 #include "stage_warp.hpp"
 
 using namespace h3c;
@@ -123,6 +124,10 @@ struct h3c_solver_s {
   size_t halo_smem = 0;
   double halo_mean = 0;
   int halo_maxh = 0;
+  // split tile kernel (h3c_stage_split.cu), the Euler/AUSM default: packed slots, shared memory
+  bool split_ok = false;
+  void* d_pack = nullptr;
+  size_t split_smem = 0;
   // CNS tile kernel (h3c_stage_cns.cu): its tables reuse d_lnb / d_hids / d_hoff
   bool cns_ok = false;
   int* d_h1end = nullptr;
@@ -212,7 +217,9 @@ void free_grid(h3c_solver s) {
   dfree(s->d_blk_inst); dfree(s->d_inst_end); dfree(s->d_ginst);
   dfree(s->d_lnb); dfree(s->d_hids); dfree(s->d_hoff); dfree(s->d_goff); dfree(s->d_grp);
   dfree(s->d_h1end); dfree(s->d_hnb); dfree(s->d_gsl);
+  dfree(s->d_pack);
   s->halo_ok = false;
+  s->split_ok = false;
   s->cns_ok = false;
   dfree(s->d_adj);
   s->adj_cap = 0;
@@ -435,6 +442,15 @@ void stage_t(h3c_solver s, const double* qin, double* out) {
       return;
     }
   }
+  if (PHYS == EULER && FLUX == AUSM && s->tile && s->split_ok) {
+    const long long grid = s->persist_blocks > 0 ? std::min<long long>(s->persist_blocks, s->ntiles) : s->ntiles;
+    const SplitGeom sg{(const uint4*)s->d_pack, (const uint2*)s->d_pack,
+                       HaloGeom{s->d_lnb, s->d_hids, s->d_hoff, s->d_grp, s->d_goff, 0}};
+    split_stage(ND, std::is_same<R, float>::value, MODE, HANG, FUSE, qin, out, geometry(s), sg, s->pc, s->d_sc,
+                &s->d_sc->dtmin_ord, (unsigned)std::max<long long>(1, grid), s->split_smem, s->stream);
+    return;
+  }
+  // tables beyond the slots' 15 or the cell ids' 29 bits: the per-lane tile kernel, which needs none
   if (PHYS == EULER && FLUX == AUSM && s->tile) {
     constexpr size_t smem = ausm_smem_bytes<R, ND>();
     static bool attr = false;  // one opt-in per instantiation (dynamic smem above 48 KB)
@@ -783,8 +799,8 @@ __global__ void k_check_tables(const int* __restrict__ nbr, const int* __restric
     for (int j = 0; j < nsubc; ++j) b += !(sub[j * nsub + i] >= 0 && sub[j * nsub + i] < n_tot);
   if (i < ng) b += !(gbndry[i] >= 0 && gbndry[i] < n_int);
   if (i < nhids) {
-    const int h = hids[i] & hid_mask;
-    b += !(hids[i] >= 0 && h < n_tot);
+    const int h = hids[i] & hid_mask;  // Euler entries: without their direction and side bits
+    b += !(h >= 0 && h < n_tot);
   }
   if (b) atomicAdd(bad, b);
 }
@@ -1015,7 +1031,9 @@ static int set_grids(h3c_solver s, int ninst, const h3c_grid* grids) {
     if (s->halo_cap > 0) HH.hmax = std::min(HH.hmax, s->halo_cap);
     const size_t smem = halo_smem_bytes(nd, mixed, HH.hmax);
     const int bps = halo_prepare(nd, mixed, smem);
-    if (bps > 0) {
+    const size_t ssmem = split_smem_bytes(nd, mixed);
+    const bool split = split_prepare(nd, mixed, ssmem);
+    if (bps > 0 || split) {
       H3C_CUDA(s, cudaMalloc(&s->d_lnb, sizeof(unsigned short) * HH.lnb.size()));
       H3C_CUDA(s, cudaMalloc(&s->d_hids, sizeof(int) * HH.ids.size()));
       H3C_CUDA(s, cudaMalloc(&s->d_hoff, sizeof(int) * HH.off.size()));
@@ -1031,7 +1049,12 @@ static int set_grids(h3c_solver s, int ninst, const h3c_grid* grids) {
       s->halo_bps = bps;
       s->halo_mean = HH.mean_halo;
       s->halo_maxh = HH.max_halo;
-      s->halo_ok = true;
+      s->halo_ok = bps > 0;
+      if (split) {
+        H3C_CUDA(s, cudaMalloc(&s->d_pack, split_pack_bytes(nd, L)));
+        s->split_smem = ssmem;
+        s->split_ok = true;
+      }
     }
   }
   if (s->desc.physics == H3C_EULER && s->desc.flux == H3C_FLUX_AUSM && s->desc.reconstruction != H3C_RECON_MUSCL)
@@ -1075,13 +1098,14 @@ static int set_grids(h3c_solver s, int ninst, const h3c_grid* grids) {
   // return before its DMA lands, a cudaMemset before it runs): finish them
   // before the stream's kernels read the tables.
   H3C_CUDA(s, cudaStreamSynchronize(cudaStreamLegacy));
+  if (s->split_ok) split_pack(nd, s->d_lnb, s->d_lvl, L, L, s->d_pack, s->stream);
   {
     unsigned long long* d_bad = nullptr;
     H3C_CUDA(s, cudaMalloc(&d_bad, sizeof(unsigned long long)));
     H3C_CUDA(s, cudaMemsetAsync(d_bad, 0, sizeof(unsigned long long), s->stream));
-    const long long nh = (s->halo_ok || s->cns_ok) && s->d_hids ? HH.ids.size() + CH.base.ids.size() : 0;
+    const long long nh = s->d_hids ? HH.ids.size() + CH.base.ids.size() : 0;
     const long long span = std::max({n_int, nsub, ng, nh, 1LL});
-    const int hid_mask = s->halo_ok ? kHaloCellMask : -1;  // Euler entries carry a direction
+    const int hid_mask = halo_tables ? kHaloCellMask : -1;  // Euler entries carry a direction and a side
     k_check_tables<<<blocks(span), kBlock, 0, s->stream>>>(s->d_nbr, s->d_sub, s->d_gbndry, s->d_lvl, s->d_hids,
                                                            hid_mask, nh, s->d_dev2caller, n_int, n_tot, L, nsub,
                                                            np, nsubc, ng,

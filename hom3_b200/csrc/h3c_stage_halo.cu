@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kHaloTile, 3)
 #pragma unroll
         for (int v = 0; v < NV; ++v) qh[v] = land[(size_t)v * S + TB + h];
         face_state_of<R, ND>(qh, gamma, gm1, th, ph, Mh);
-        const int dir = hid[k] >> kHaloDirShift;
+        const int dir = halo_dir(hid[k]);
         R Md = Mh[0];
 #pragma unroll
         for (int d = 1; d < ND; ++d) Md = dir == d ? Mh[d] : Md;
@@ -342,7 +342,7 @@ bool halo_build(int nd, long long ld, long long ntiles, const std::vector<long l
   std::vector<std::vector<unsigned short>> grp(ntiles);
   std::atomic<bool> ok{true};
   auto work = [&](long long t0, long long t1) {
-    std::vector<long long> tmp;  // (cell << 2) | direction
+    std::vector<long long> tmp;  // (cell << 3) | position (2 direction + side)
     for (long long t = t0; t < t1 && ok.load(std::memory_order_relaxed); ++t) {
       const long long c0 = t * TB, ce = tile_end[t];
       auto outside = [&](long long v) { return v < c0 || v >= ce; };
@@ -350,14 +350,13 @@ bool halo_build(int nd, long long ld, long long ntiles, const std::vector<long l
       for (long long c = c0; c < ce; ++c)
         for (int p = 0; p < NP; ++p) {
           const long long v = nbr[p * ld + c];
-          const int dir = p >> 1;
           if (v >= 0) {
-            if (outside(v)) tmp.push_back((v << 2) | dir);
+            if (outside(v)) tmp.push_back((v << 3) | p);
           } else if (v <= -2) {
             const long long k = -v - 2;
             for (int j = 0; j < NS; ++j) {
               const long long sv = sub[j * nsub + k];
-              if (outside(sv)) tmp.push_back((sv << 2) | dir);
+              if (outside(sv)) tmp.push_back((sv << 3) | p);
             }
           }
         }
@@ -367,18 +366,17 @@ bool halo_build(int nd, long long ld, long long ntiles, const std::vector<long l
         ok = false;
         break;
       }
-      auto slot = [&](long long v, int dir) -> unsigned short {
+      auto slot = [&](long long v, int p) -> unsigned short {
         if (!outside(v)) return (unsigned short)(v - c0);
-        return (unsigned short)(TB + (std::lower_bound(tmp.begin(), tmp.end(), (v << 2) | dir) - tmp.begin()));
+        return (unsigned short)(TB + (std::lower_bound(tmp.begin(), tmp.end(), (v << 3) | p) - tmp.begin()));
       };
       std::vector<unsigned short>& G = grp[t];
       for (long long c = c0; c < ce; ++c)
         for (int p = 0; p < NP; ++p) {
           const long long v = nbr[p * ld + c];
-          const int dir = p >> 1;
           unsigned short e = 0;
           if (v >= 0) {
-            e = slot(v, dir);
+            e = slot(v, p);
           } else if (v <= -2) {
             const long long k = -v - 2;
             const size_t gi = G.size() / NS;
@@ -387,13 +385,16 @@ bool halo_build(int nd, long long ld, long long ntiles, const std::vector<long l
               break;
             }
             e = (unsigned short)(kGroupBit | gi);
-            for (int j = 0; j < NS; ++j) G.push_back(slot(sub[j * nsub + k], dir));
+            for (int j = 0; j < NS; ++j) G.push_back(slot(sub[j * nsub + k], p));
           }
           H.lnb[(size_t)p * ld + c] = e;
         }
       std::vector<int>& hl = halo[t];
       hl.resize(tmp.size());
-      for (size_t i = 0; i < tmp.size(); ++i) hl[i] = (int)((tmp[i] >> 2) | ((tmp[i] & 3) << kHaloDirShift));
+      for (size_t i = 0; i < tmp.size(); ++i) {
+        const unsigned p = tmp[i] & 7;
+        hl[i] = (int)((unsigned)(tmp[i] >> 3) | ((p >> 1) << kHaloDirShift) | ((p & 1) << 31));
+      }
     }
   };
   const int nthr = std::max(1, std::min<int>((int)std::thread::hardware_concurrency(), 16));

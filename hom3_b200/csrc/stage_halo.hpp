@@ -4,10 +4,10 @@
 // The kernel replaces hom3's num_flux + evolve loop (src/solver/fv/
 // solver.hpp:440-460, 470-494) for Euler with the AUSM flux.  It works on
 // 256-cell tiles of the Morton order.  Per tile, set-up time tables list
-//   * the tile's halo: every (cell, direction) pair such that a face of a
-//     tile cell along that direction reads a cell outside the tile
-//     (same-level neighbours, ghosts and the fine cells of coarse/fine
-//     sub-face groups), sorted, and
+//   * the tile's halo: every (cell, direction, side) triple such that a face
+//     of a tile cell along that direction reads a cell outside the tile on
+//     that side (same-level neighbours, ghosts and the fine cells of
+//     coarse/fine sub-face groups), sorted, and
 //   * for every cell and face position the shared-memory slot the face's
 //     neighbour lives in (0..255: a tile cell, 256 + h: halo cell h) or, with
 //     kGroupBit set, the index of the face's sub-face group in the tile's
@@ -25,11 +25,14 @@ namespace h3c {
 constexpr int kHaloTile = 256;              // cells per tile = threads per block
 constexpr int kHaloMaxSlots = 1024;         // halo entries a tile may hold in shared memory
 constexpr unsigned short kGroupBit = 0x8000;
-// Euler halo entries are (cell, direction) pairs: the id word carries the
-// cell in its low 29 bits and the face direction it is read across above
-// them (the CNS tables list plain cell ids).
+// Euler halo entries are (cell, direction, side) triples: the id word carries
+// the cell in its low 29 bits, the face direction it is read across in bits
+// 29-30 and in bit 31 whether it lies on the plus side of that face (the CNS
+// tables list plain cell ids).
 constexpr int kHaloDirShift = 29;
 constexpr int kHaloCellMask = (1 << kHaloDirShift) - 1;
+__host__ __device__ inline int halo_dir(int id) { return (id >> kHaloDirShift) & 3; }
+__host__ __device__ inline bool halo_plus(int id) { return id < 0; }
 
 // Device tables of the halo-staged kernel.
 struct HaloGeom {
@@ -55,7 +58,7 @@ struct HaloHost {
 // tiles of [0, n_int); tile_end[t] is the end of tile t's cells (tiles never
 // span two batch instances).  Returns false when a tile's slots overflow 15
 // bits or the cells 29 bits (the caller then keeps the per-lane tile kernel).
-// Halo ids carry the direction in bits 29-30.
+// Halo ids carry the direction in bits 29-30, the side in bit 31.
 bool halo_build(int nd, long long ld, long long ntiles, const std::vector<long long>& tile_end, const int* nbr,
                 const int* sub, long long nsub, HaloHost& H);
 
