@@ -40,6 +40,20 @@ struct Scalars {
   long long mindt_ord;  // min of cell dt for h3c_min_dt
   int status;           // kStatus* bits, sticky until h3c_status reads them
   int pad;
+  struct HostScalars* mirror;  // instance 0: the host's copy of the step scalars (mapped pinned memory), or nullptr
+};
+
+// What h3c_dt / h3c_time / h3c_step read.  The first kernel of a step writes
+// it over PCIe while the step runs (time and step as they are after the
+// step), so reading it after the stream is synchronised needs no copy of its
+// own.  A cell check that fails later in the step sets its own word: single
+// stores, since host memory takes no atomics from every device.
+struct HostScalars {
+  double dt, time;
+  long long step;
+  int status;     // bits as the step began
+  int bad_state;  // the step's own findings
+  int timeout;
 };
 
 // Scalars::status bits
@@ -83,6 +97,8 @@ struct Geometry {
   long long ntiles;
   // advection velocity u(x_center) of every cell, ghosts included: [nd][ld] (nullptr otherwise)
   const double* __restrict__ vel;
+  // start state of the step, which the later Runge-Kutta stages combine with (may be the stage's own output)
+  const double* q0;
 };
 
 __device__ __forceinline__ int tile_instance(const Geometry& g, long long tile) {
@@ -175,8 +191,28 @@ __device__ __forceinline__ void block_min_atomic_nobar(long long v, long long* d
 // Records in the instance's status that some cell of this warp failed the
 // state check (one atomic per warp that saw one; every lane must call).
 __device__ __forceinline__ void flag_bad_state(bool bad, const Scalars* sc, int inst) {
-  if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0)
+  if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) {
     atomicOr(const_cast<int*>(&sc[inst].status), kStatusState);
+    if (sc[inst].mirror) *(volatile int*)&sc[inst].mirror->bad_state = 1;
+  }
+}
+// Records that a bounded wait ran out (one thread calls).
+__device__ __forceinline__ void flag_timeout(const Scalars* sc, int* status) {
+  atomicOr(status, kStatusTimeout);
+  if (sc->mirror) *(volatile int*)&sc->mirror->timeout = 1;
+}
+
+// Programmatic dependent launch: the next kernel of the stream may be set up
+// while this one still runs; it waits here, before it touches memory, until
+// every kernel before it has finished and its writes are visible.  The steps of
+// small grids are chains of kernels of a few microseconds, whose launch gaps
+// this hides (with the scalar work moved into the conditions' kernel, see
+// StepBegin: 256^2 MUSCL, SSP-RK3, 30 steps 2187 -> 1465 us; 48 coupled
+// 512 x 192 steps 2458 -> 1481 us).  Every kernel launched that way starts
+// with this call.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
 }
 
 // ---------------------------------------------------------------------------
@@ -445,12 +481,8 @@ __global__ void __launch_bounds__(kBlock) k_cfl(const double* __restrict__ q, Ge
   block_min_atomic(o, per_instance(dst, inst));
 }
 
-#ifndef H3C_DEVICE_FUNCTIONS_ONLY  // non-template kernels: defined in one translation unit
 // set_dt: solver.hpp:541-551 (dtmin_ord holds compute_dt of the current lhs)
-__global__ void k_set_dt(Scalars* s0, int reset_after, int n_inst) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_inst) return;
-  Scalars* s = s0 + i;
+__device__ __forceinline__ void set_dt(Scalars* s, bool reset_after) {
   double dt;
   if (s->time + s->dt < s->tEnd) {
     dt = (s->step == s->forced_step) ? s->forced_dt : ord_to_dbl(s->dtmin_ord);
@@ -460,6 +492,73 @@ __global__ void k_set_dt(Scalars* s0, int reset_after, int n_inst) {
   s->dt = dt;
   if (!(dt >= 1e-300 && dt <= 1e300)) s->status |= kStatusDt;  // utilities.hpp:74-76
   if (reset_after) s->dtmin_ord = kOrdMax;
+}
+
+// The scalar work of a step, done by one block of the kernel that applies
+// the step's first conditions: set_dt, and -- the stages read dt alone --
+// advance (solver.hpp:502-505) right after it.  Two kernels of one thread
+// each per step otherwise, which the runs of small grids spent as much on as
+// on their cells; and the host's copy of the scalars is written on the way
+// (64 x 64 Euler with dt read after every step, 10 steps: 340 -> 220 us).
+struct StepBegin {
+  Scalars* sc = nullptr;      // nullptr: no scalar work
+  int n_inst = 1;
+  int advance = 0;            // time and step as after the step (no later part reads the time)
+  const double* from = nullptr;  // frozen steps: the step's dt is from[idx]
+  double* record = nullptr;   // records the step's dt at idx
+  long long idx = 0;
+  // the coupled loop (coupling.hpp:52-63): both solvers' dt from both minima
+  Scalars* heat = nullptr;
+  double scaling = 1.0;
+  double* heat_record = nullptr;
+};
+
+__device__ __forceinline__ void advance_scalars(Scalars* s) {
+  s->time += s->dt;
+  s->step += 1;
+  if (s->mirror) {
+    volatile HostScalars* m = s->mirror;
+    m->dt = s->dt;
+    m->time = s->time;
+    m->step = s->step;
+    m->status = s->status;
+    m->bad_state = 0;
+    m->timeout = 0;
+  }
+}
+
+__device__ __forceinline__ void step_begin(const StepBegin& b) {
+  for (int i = threadIdx.x; i < b.n_inst; i += blockDim.x) {
+    Scalars* s = b.sc + i;
+    if (b.heat) {
+      Scalars* h = b.heat;
+      const double min_dt_cns = ord_to_dbl(s->dtmin_ord);
+      const double min_dt_heat = ord_to_dbl(h->dtmin_ord) / b.scaling;
+      const double dt = (min_dt_heat < min_dt_cns) ? min_dt_heat : min_dt_cns;  // std::min
+      s->forced_step = s->step;
+      s->forced_dt = dt;
+      h->forced_step = h->step;
+      h->forced_dt = dt * b.scaling;
+      set_dt(h, true);
+      if (b.heat_record) b.heat_record[b.idx] = h->dt;
+      advance_scalars(h);
+    }
+    if (b.from) s->dt = b.from[b.idx];
+    else set_dt(s, true);
+    if (b.record) b.record[b.idx] = s->dt;
+    if (b.advance) advance_scalars(s);
+  }
+}
+
+#ifndef H3C_DEVICE_FUNCTIONS_ONLY  // non-template kernels: defined in one translation unit
+__global__ void k_set_dt(Scalars* s0, int reset_after, int n_inst) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n_inst) set_dt(s0 + i, reset_after);
+}
+// a step's scalar work where no conditions are applied
+__global__ void __launch_bounds__(kBlock) k_step_begin(StepBegin b) {
+  chain_begin();
+  step_begin(b);
 }
 // advance: solver.hpp:502-505
 __global__ void k_advance(Scalars* s0, int n_inst) {
@@ -523,9 +622,18 @@ __device__ __forceinline__ double partner_T(const BcParam& B, const PartnerView&
 template <int ND, int PHYS>
 __global__ void __launch_bounds__(kBlock) k_bc(double* __restrict__ q, const double* __restrict__ qlhs,
                                                Geometry g, GhostTables gt, PhysConst pc,
-                                               const Scalars* __restrict__ sc, PartnerView pv) {
+                                               const Scalars* sc, PartnerView pv, StepBegin begin) {
   constexpr int NV = nvars<ND, PHYS>();
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  chain_begin();
+  unsigned blk = blockIdx.x;
+  if (begin.sc) {  // the first block does the step's scalar work; no condition launched with it reads the scalars
+    if (blk == 0) {
+      step_begin(begin);
+      return;
+    }
+    --blk;
+  }
+  const long long i = (long long)blk * blockDim.x + threadIdx.x;
   if (i >= gt.ng) return;
   const int b = gt.bc_apply[i];
   if (b == 255) return;
@@ -685,6 +793,7 @@ template <int ND>
 __global__ void __launch_bounds__(kBlock) k_slopes(const double* __restrict__ q, Geometry g, GhostTables gt,
                                                    double* __restrict__ sl) {
   constexpr int NV = ND + 2;
+  chain_begin();
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= g.n_tot) return;
   const long long ld = g.ld;
@@ -713,8 +822,8 @@ __global__ void __launch_bounds__(kBlock) k_slopes(const double* __restrict__ q,
   }
 }
 
-// Explicit stage update from q0 (the step's start state, in `out` for the
-// in-place stages), the stage input qc and r = dt/dx R(qc):
+// Explicit stage update from q0 (the step's start state), the stage input qc
+// and r = dt/dx R(qc):
 //   MODE 0: qc + r (FE, first stage of RK2 / SSP-RK3)
 //   MODE 2: 0.5 ((q0 + qc) + r) (RK2 second stage, solver.hpp:483-494)
 //   MODE 3: 3/4 q0 + 1/4 (qc + r), MODE 4: 1/3 q0 + 2/3 (qc + r) (EXTENSION: SSP-RK3)
@@ -728,8 +837,8 @@ template <int MODE> __device__ __forceinline__ double rk_combine(double q0, doub
 // ---------------------------------------------------------------------------
 // Stage kernel: num_flux (solver.hpp:440-460) + the explicit update of evolve
 // (solver.hpp:470-494).
-//   out = rk_combine<MODE>(out, qin, dt/dx R(qin)); MODE 2, 3 and 4 read the
-//   start state from `out` (in place).
+//   out = rk_combine<MODE>(q0, qin, dt/dx R(qin)); MODE 2, 3 and 4 read the
+//   step's start state q0 = Geometry::q0 (`out` itself for an in-place stage).
 // FUSE: also reduce the next step's cell dt of `out` into *dtmin (the
 // compute_dt of the next set_dt; valid when no condition rewrites interior cells).
 // HANG: the grid has coarse/fine faces (EXTENSION, not in hom3).
@@ -739,6 +848,7 @@ __global__ void __launch_bounds__(kBlock) k_stage(const double* __restrict__ qin
                                                   const double* __restrict__ sl, Geometry g, PhysConst pc,
                                                   const Scalars* __restrict__ sc, long long* dtmin) {
   constexpr int NV = nvars<ND, PHYS>();
+  chain_begin();
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int inst = tile_instance(g, blockIdx.x);
   const bool live = c < instance_end(g, inst);
@@ -949,7 +1059,7 @@ __global__ void __launch_bounds__(kBlock) k_stage(const double* __restrict__ qin
     const double k = dt / dx;
     double o[NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) o[v] = rk_combine<MODE>(MODE == 0 ? 0.0 : out[v * ld + c], qc[v], k * acc[v]);
+    for (int v = 0; v < NV; ++v) o[v] = rk_combine<MODE>(MODE == 0 ? 0.0 : g.q0[v * ld + c], qc[v], k * acc[v]);
 #pragma unroll
     for (int v = 0; v < NV; ++v) out[v * ld + c] = o[v];
     if (FUSE) {
@@ -1132,7 +1242,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_stage_tile(const double* __restri
     const double k = dt / dx;
     double o[NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) o[v] = rk_combine<MODE>(MODE == 0 ? 0.0 : out[v * ld + c], qc[v], k * acc[v]);
+    for (int v = 0; v < NV; ++v) o[v] = rk_combine<MODE>(MODE == 0 ? 0.0 : g.q0[v * ld + c], qc[v], k * acc[v]);
 #pragma unroll
     for (int v = 0; v < NV; ++v) out[v * ld + c] = o[v];
     if (FUSE) {
@@ -1220,7 +1330,7 @@ __global__ void __launch_bounds__(TB, H3C_AUSM_MINB * kBlock / TB) k_stage_ausm(
     const int inst = tile_instance(g, tile);
     const long long tile_end = min(c0 + (long long)TB, instance_end(g, inst));
     const bool live = c < tile_end;
-    if (MODE != 0 && live) prefetch_row_l2<NV>(out, ld, c);  // the in-place start state, read at the update
+    if (MODE != 0 && live) prefetch_row_l2<NV>(g.q0, ld, c);  // the start state, read at the update
 
     // ---- own loads first: state, neighbours, level ----
     double qc[NV];
@@ -1350,7 +1460,7 @@ __global__ void __launch_bounds__(TB, H3C_AUSM_MINB * kBlock / TB) k_stage_ausm(
       double qo[NV];
       if (MODE != 0) {
 #pragma unroll
-        for (int v = 0; v < NV; ++v) qo[v] = out[v * ld + c];
+        for (int v = 0; v < NV; ++v) qo[v] = g.q0[v * ld + c];
       }
       // the cell's own state and length read again (L1/L2) rather than held
       // in registers across the face loops: fewer spills at 64 registers
@@ -1400,7 +1510,7 @@ __global__ void __launch_bounds__(kBlock, H3C_CELL_MINB) k_stage_ausm_cell(const
   const bool live = c < instance_end(g, inst);
   const long long ld = g.ld;
   const R gamma = (R)pc.gamma, gm1 = (R)pc.gm1;
-  if (MODE != 0 && live) prefetch_row_l2<NV>(out, ld, c);  // the in-place start state, read at the update
+  if (MODE != 0 && live) prefetch_row_l2<NV>(g.q0, ld, c);  // the start state, read at the update
   // The cell's own face state (theta, p, Mach number along each direction),
   // kept in the thread's column of shared memory rather than in registers
   // across the direction loop: at three blocks per SM the loop spills otherwise.
@@ -1520,7 +1630,7 @@ __global__ void __launch_bounds__(kBlock, H3C_CELL_MINB) k_stage_ausm_cell(const
     for (int v = 0; v < NV; ++v) qc[v] = __ldg(qin + v * ld + c);
     if (MODE != 0) {
 #pragma unroll
-      for (int v = 0; v < NV; ++v) qo[v] = out[v * ld + c];
+      for (int v = 0; v < NV; ++v) qo[v] = g.q0[v * ld + c];
     }
     double o[NV];
 #pragma unroll

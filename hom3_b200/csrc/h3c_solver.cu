@@ -30,6 +30,7 @@
 #include "muscl_kernels.cuh"
 #include "muscl_adjoint.cuh"
 #include "cns_adjoint.cuh"
+#include "launch.hpp"
 #include "stage_halo.hpp"
 #include "stage_split.hpp"
 #include "stage_warp.hpp"
@@ -84,6 +85,7 @@ struct h3c_solver_s {
   unsigned char *d_gpos = nullptr, *d_gapply = nullptr, *d_gown = nullptr;
   double* d_gdx = nullptr;
   int* d_gpartner = nullptr;
+  int* d_gsrc = nullptr;  // per ghost the cell whose MUSCL gradient it takes (periodic: its paired cell, else itself)
   double* d_xc = nullptr;
   double* d_vel = nullptr;  // advection velocity [nd][ld], internal numbering, ghosts included
   bool vel_set = false;
@@ -104,9 +106,13 @@ struct h3c_solver_s {
   std::vector<long long> dev2caller, caller2dev;
   Scalars* d_sc = nullptr;
   Scalars* h_sc = nullptr;  // pinned host copy of instance 0's scalars (the per-step dt read-back)
+  HostScalars* h_mirror = nullptr;  // what the steps' kernels write of them (mapped pinned memory)
+  bool mirror_valid = false;        // the last thing that changed the scalars was a step that wrote the mirror
+  const double* stage_q0 = nullptr; // start state of the stage being launched (Geometry::q0)
   bool unfused_dt = false;  // a condition rewrites interior cells (vortex)
   bool ghost_unapplied = false;  // some ghost gets no condition (hom3's find_if segments)
   bool needs_partner = false, needs_periodic = false;  // coupling / periodic conditions present
+  bool has_exchange = false;  // ghosts the caller writes between the parts of a step
   bool partner_set = false, periodic_set = false;
   bool tile = true;  // Euler stages use the shared-memory tile kernel
   bool cns_adj_dual = false;  // CNS adjoint faces by dual numbers instead of the hand-written reverse
@@ -218,6 +224,8 @@ void free_grid(h3c_solver s) {
   dfree(s->d_lnb); dfree(s->d_hids); dfree(s->d_hoff); dfree(s->d_goff); dfree(s->d_grp);
   dfree(s->d_h1end); dfree(s->d_hnb); dfree(s->d_gsl);
   dfree(s->d_pack);
+  dfree(s->d_gsrc);
+  s->mirror_valid = false;
   s->halo_ok = false;
   s->split_ok = false;
   s->cns_ok = false;
@@ -241,6 +249,7 @@ Geometry geometry(const h3c_solver s) {
   g.inst_end = s->n_inst > 1 ? s->d_inst_end : nullptr;
   g.ntiles = s->ntiles;
   g.vel = s->d_vel;
+  g.q0 = s->stage_q0;
   return g;
 }
 
@@ -309,25 +318,33 @@ struct Launch {
 
 // ---- kernel dispatch -------------------------------------------------------
 template <int ND, int PHYS>
-void launch_bc_t(h3c_solver s, double* q, const double* qlhs) {
+void launch_bc_t(h3c_solver s, double* q, const double* qlhs, const StepBegin& begin) {
   PartnerView pv{nullptr, 0};
   if (s->partner) pv = PartnerView{s->partner_override ? s->partner_override : s->partner->d_q[0], s->partner->ld};
   Launch L(s, K_BC);
-  k_bc<ND, PHYS><<<blocks(s->ng), kBlock, 0, s->stream>>>(q, qlhs, geometry(s), ghosts(s), s->pc, s->d_sc, pv);
+  launch_chain(k_bc<ND, PHYS>, blocks(s->ng) + (begin.sc ? 1 : 0), kBlock, 0, s->stream, q, qlhs, geometry(s), ghosts(s),
+               s->pc, s->d_sc, pv, begin);
 }
-// conditions applied to q; coupling conditions read temperatures from qlhs
-void launch_bc_ptr(h3c_solver s, double* q, const double* qlhs) {
-  if (s->ng == 0) return;
+// conditions applied to q; coupling conditions read temperatures from qlhs;
+// begin: the step's scalar work, done by the same launch
+void launch_bc_ptr(h3c_solver s, double* q, const double* qlhs, const StepBegin& begin = StepBegin{}) {
+  if (s->ng == 0) {
+    if (begin.sc) {
+      Launch L(s, K_SCALAR);
+      launch_chain(k_step_begin, 1, kBlock, 0, s->stream, begin);
+    }
+    return;
+  }
   if (s->nd == 2) {
-    if (s->desc.physics == H3C_EULER) launch_bc_t<2, EULER>(s, q, qlhs);
-    else if (s->desc.physics == H3C_CNS) launch_bc_t<2, CNS>(s, q, qlhs);
-    else if (s->desc.physics == H3C_ADVECTION) launch_bc_t<2, ADVECTION>(s, q, qlhs);
-    else launch_bc_t<2, HEAT>(s, q, qlhs);
+    if (s->desc.physics == H3C_EULER) launch_bc_t<2, EULER>(s, q, qlhs, begin);
+    else if (s->desc.physics == H3C_CNS) launch_bc_t<2, CNS>(s, q, qlhs, begin);
+    else if (s->desc.physics == H3C_ADVECTION) launch_bc_t<2, ADVECTION>(s, q, qlhs, begin);
+    else launch_bc_t<2, HEAT>(s, q, qlhs, begin);
   } else {
-    if (s->desc.physics == H3C_EULER) launch_bc_t<3, EULER>(s, q, qlhs);
-    else if (s->desc.physics == H3C_CNS) launch_bc_t<3, CNS>(s, q, qlhs);
-    else if (s->desc.physics == H3C_ADVECTION) launch_bc_t<3, ADVECTION>(s, q, qlhs);
-    else launch_bc_t<3, HEAT>(s, q, qlhs);
+    if (s->desc.physics == H3C_EULER) launch_bc_t<3, EULER>(s, q, qlhs, begin);
+    else if (s->desc.physics == H3C_CNS) launch_bc_t<3, CNS>(s, q, qlhs, begin);
+    else if (s->desc.physics == H3C_ADVECTION) launch_bc_t<3, ADVECTION>(s, q, qlhs, begin);
+    else launch_bc_t<3, HEAT>(s, q, qlhs, begin);
   }
 }
 void launch_bc(h3c_solver s, int which) { launch_bc_ptr(s, s->d_q[which], s->d_q[0]); }
@@ -339,6 +356,7 @@ void launch_cfl_t(h3c_solver s, long long* slot) {
 }
 void launch_cfl(h3c_solver s, long long* slot) {
   if (s->desc.physics == H3C_ADVECTION && !s->vel_set) return;  // no velocity yet: no time step
+  s->mirror_valid = false;  // the pass checks every cell
   {
     Launch L(s, K_SCALAR);
     k_reset_slot<<<blocks(s->n_inst), kBlock, 0, s->stream>>>(slot, s->n_inst);
@@ -358,32 +376,23 @@ void launch_cfl(h3c_solver s, long long* slot) {
 
 void launch_slopes_ptr(h3c_solver s, const double* q) {
   Launch L(s, K_SLOPES);
-  if (s->nd == 2)
-    k_slopes<2><<<blocks(s->n_tot), kBlock, 0, s->stream>>>(q, geometry(s), ghosts(s), s->d_slopes);
-  else
-    k_slopes<3><<<blocks(s->n_tot), kBlock, 0, s->stream>>>(q, geometry(s), ghosts(s), s->d_slopes);
+  launch_chain(s->nd == 2 ? k_slopes<2> : k_slopes<3>, blocks(s->n_tot), kBlock, 0, s->stream, q, geometry(s), ghosts(s),
+               s->d_slopes);
 }
 
-void launch_slopes(h3c_solver s, int which) {
-  Launch L(s, K_SLOPES);
-  if (s->nd == 2)
-    k_slopes<2><<<blocks(s->n_tot), kBlock, 0, s->stream>>>(s->d_q[which], geometry(s), ghosts(s), s->d_slopes);
-  else
-    k_slopes<3><<<blocks(s->n_tot), kBlock, 0, s->stream>>>(s->d_q[which], geometry(s), ghosts(s), s->d_slopes);
-}
+void launch_slopes(h3c_solver s, int which) { launch_slopes_ptr(s, s->d_q[which]); }
 
 // EXTENSION: limited least-squares gradients of the stage input (MUSCL)
-void launch_grad(h3c_solver s, const double* q) {
+// ghosts_too: the periodic ghosts' copies as well (the adjoint reads them; the stage reads through d_gsrc)
+void launch_grad(h3c_solver s, const double* q, bool ghosts_too) {
   Launch L(s, K_SLOPES);
   const double K = s->desc.limiter_k;
-  if (s->nd == 2) {
-    if (s->nsub > 0) k_muscl_grad<2, true><<<blocks(s->n_int), kBlock, 0, s->stream>>>(q, s->d_xc, geometry(s), s->pc, K, s->d_slopes);
-    else k_muscl_grad<2, false><<<blocks(s->n_int), kBlock, 0, s->stream>>>(q, s->d_xc, geometry(s), s->pc, K, s->d_slopes);
-    if (s->needs_periodic) k_muscl_ghosts<2><<<blocks(s->ng), kBlock, 0, s->stream>>>(s->d_slopes, geometry(s), ghosts(s));
-  } else {
-    if (s->nsub > 0) k_muscl_grad<3, true><<<blocks(s->n_int), kBlock, 0, s->stream>>>(q, s->d_xc, geometry(s), s->pc, K, s->d_slopes);
-    else k_muscl_grad<3, false><<<blocks(s->n_int), kBlock, 0, s->stream>>>(q, s->d_xc, geometry(s), s->pc, K, s->d_slopes);
-    if (s->needs_periodic) k_muscl_ghosts<3><<<blocks(s->ng), kBlock, 0, s->stream>>>(s->d_slopes, geometry(s), ghosts(s));
+  const auto grad = s->nd == 2 ? (s->nsub > 0 ? k_muscl_grad<2, true> : k_muscl_grad<2, false>)
+                               : (s->nsub > 0 ? k_muscl_grad<3, true> : k_muscl_grad<3, false>);
+  launch_chain(grad, blocks(s->n_int), kBlock, 0, s->stream, q, s->d_xc, geometry(s), s->pc, K, s->d_slopes);
+  if (ghosts_too && s->needs_periodic) {
+    if (s->nd == 2) k_muscl_ghosts<2><<<blocks(s->ng), kBlock, 0, s->stream>>>(s->d_slopes, geometry(s), ghosts(s));
+    else k_muscl_ghosts<3><<<blocks(s->ng), kBlock, 0, s->stream>>>(s->d_slopes, geometry(s), ghosts(s));
   }
 }
 
@@ -391,8 +400,8 @@ template <int ND, int PHYS, int FLUX, class R, int MODE, bool HANG, bool FUSE>
 void stage_t(h3c_solver s, const double* qin, double* out) {
   Launch L(s, MODE == 0 ? K_STAGE1 : K_STAGE2);
   if (PHYS == EULER && FLUX == AUSM && s->desc.reconstruction == H3C_RECON_MUSCL) {
-    k_stage_muscl<ND, R, MODE, HANG, FUSE><<<blocks(s->n_int), kBlock, 0, s->stream>>>(
-        qin, out, s->d_slopes, s->d_xc, geometry(s), s->pc, s->d_sc, &s->d_sc->dtmin_ord);
+    launch_chain(k_stage_muscl<ND, R, MODE, HANG, FUSE>, blocks(s->n_int), kBlock, 0, s->stream, qin, out, s->d_slopes,
+                 s->d_xc, geometry(s), s->pc, s->d_sc, &s->d_sc->dtmin_ord, s->needs_periodic ? s->d_gsrc : nullptr);
     return;
   }
   if (PHYS == CNS && s->tile && s->halo && s->cns_ok) {
@@ -476,8 +485,8 @@ void stage_t(h3c_solver s, const double* qin, double* out) {
         qin, out, geometry(s), s->pc, s->d_sc, &s->d_sc->dtmin_ord);
     return;
   }
-  k_stage<ND, PHYS, FLUX, R, MODE, HANG, FUSE><<<blocks(s->n_int), kBlock, 0, s->stream>>>(
-      qin, out, s->d_slopes, geometry(s), s->pc, s->d_sc, &s->d_sc->dtmin_ord);
+  launch_chain(k_stage<ND, PHYS, FLUX, R, MODE, HANG, FUSE>, blocks(s->n_int), kBlock, 0, s->stream, qin, out,
+               s->d_slopes, geometry(s), s->pc, s->d_sc, &s->d_sc->dtmin_ord);
 }
 // Euler adjoint stage in the tile kernel (one block per Morton tile)
 template <int ND, bool HANG>
@@ -535,12 +544,14 @@ void stage_nd(h3c_solver s, int mode, const double* qin, double* out, bool fuse)
       stage_m<ND, HEAT, AUSM, double>(s, mode, qin, out, fuse);
   }
 }
-void launch_stage(h3c_solver s, int mode, const double* qin, double* out, bool fuse) {
+// out = the stage of qin; q0: the step's start state (nullptr: out holds it)
+void launch_stage(h3c_solver s, int mode, const double* qin, double* out, bool fuse, const double* q0 = nullptr) {
+  s->stage_q0 = q0 ? q0 : out;
   if (s->nd == 2) stage_nd<2>(s, mode, qin, out, fuse);
   else stage_nd<3>(s, mode, qin, out, fuse);
 }
 
-__global__ void k_init_time(Scalars* sc0, double tEnd, int n_inst) {
+__global__ void k_init_time(Scalars* sc0, double tEnd, int n_inst, HostScalars* mirror) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_inst) return;
   Scalars* sc = sc0 + i;
@@ -553,6 +564,7 @@ __global__ void k_init_time(Scalars* sc0, double tEnd, int n_inst) {
   sc->dtmin_ord = kOrdMax;
   sc->mindt_ord = kOrdMax;
   sc->status = 0;
+  sc->mirror = i == 0 ? mirror : nullptr;
 }
 __global__ void k_force_dt(Scalars* sc, double dt) {
   sc->forced_step = sc->step;
@@ -658,7 +670,15 @@ int h3c_create(const h3c_desc* d, h3c_solver* out) {
     cudaGetLastError();
     s->h_sc = nullptr;
   }
-  k_init_time<<<1, 1, 0, s->stream>>>(s->d_sc, d->time_end, 1);
+  // written by the steps' kernels through its device address (the same one under unified addressing)
+  void* mirror_dev = nullptr;
+  if (cudaHostAlloc((void**)&s->h_mirror, sizeof(HostScalars), cudaHostAllocMapped) != cudaSuccess ||
+      cudaHostGetDevicePointer(&mirror_dev, s->h_mirror, 0) != cudaSuccess || mirror_dev != (void*)s->h_mirror) {
+    cudaGetLastError();
+    if (s->h_mirror) cudaFreeHost(s->h_mirror);
+    s->h_mirror = nullptr;
+  }
+  k_init_time<<<1, 1, 0, s->stream>>>(s->d_sc, d->time_end, 1, s->h_mirror);
   *out = s.release();
   return H3C_OK;
 }
@@ -669,6 +689,7 @@ int h3c_destroy(h3c_solver s) {
   free_grid(s);
   dfree(s->d_sc);
   if (s->h_sc) cudaFreeHost(s->h_sc);
+  if (s->h_mirror) cudaFreeHost(s->h_mirror);
   for (auto& r : s->prof_rec) { cudaEventDestroy(r.second.first); cudaEventDestroy(r.second.second); }
   for (auto e : s->ev_pool) cudaEventDestroy(e);
   if (s->stream && s->own_stream) cudaStreamDestroy(s->stream);
@@ -950,7 +971,7 @@ static int set_grids(h3c_solver s, int ninst, const h3c_grid* grids) {
   s->n_bcs = (int)ubcs.size();
   s->h_bcs.assign(std::max<size_t>(1, ubcs.size()), BcParam{});
   s->unfused_dt = false;
-  s->needs_partner = s->needs_periodic = false;
+  s->needs_partner = s->needs_periodic = s->has_exchange = false;
   for (size_t q = 0; q < ubcs.size(); ++q) {
     BcParam& B = s->h_bcs[q];
     B.kind = ubcs[q].kind;
@@ -970,6 +991,7 @@ static int set_grids(h3c_solver s, int ninst, const h3c_grid* grids) {
     }
     if (B.kind >= H3C_BC_CPL_EULER_EULER && B.kind <= H3C_BC_CPL_HEAT_HEAT) s->needs_partner = true;
     if (B.kind == H3C_BC_PERIODIC) s->needs_periodic = true;
+    if (B.kind == H3C_BC_EXCHANGE) s->has_exchange = true;
   }
   if (ninst > 1 && (s->needs_partner || s->needs_periodic))
     return s->fail(H3C_E_INVALID, "h3c_set_grids: coupling and periodic conditions need a single grid");
@@ -1118,7 +1140,7 @@ static int set_grids(h3c_solver s, int ninst, const h3c_grid* grids) {
     H3C_CUDA(s, e2);
     if (bad) return s->fail(H3C_E_INVALID, "h3c_set_grid: %llu device table entries out of range", bad);
   }
-  k_init_time<<<blocks(ninst), kBlock, 0, s->stream>>>(s->d_sc, s->desc.time_end, ninst);
+  k_init_time<<<blocks(ninst), kBlock, 0, s->stream>>>(s->d_sc, s->desc.time_end, ninst, s->h_mirror);
   H3C_CUDA(s, cudaGetLastError());
   s->has_grid = true;
   return H3C_OK;
@@ -1384,7 +1406,8 @@ int h3c_reset_time(h3c_solver s) {
   if (s->ng < 0) return H3C_E_INVALID;
   if (!s->has_grid) return s->fail(H3C_E_STATE, "h3c_reset_time: no grid");
   s->stage_next = 0;  // a step run by parts starts over
-  k_init_time<<<blocks(s->n_inst), kBlock, 0, s->stream>>>(s->d_sc, s->desc.time_end, s->n_inst);
+  s->mirror_valid = false;
+  k_init_time<<<blocks(s->n_inst), kBlock, 0, s->stream>>>(s->d_sc, s->desc.time_end, s->n_inst, s->h_mirror);
   launch_cfl(s, &s->d_sc->dtmin_ord);
   k_set_dt<<<blocks(s->n_inst), kBlock, 0, s->stream>>>(s->d_sc, 0, s->n_inst);
   return s->cuda(cudaGetLastError(), "h3c_reset_time");
@@ -1405,7 +1428,7 @@ static void prepare_stage(h3c_solver s, const double* q, int which) {
   if (s->desc.physics == H3C_CNS) {
     if (!cns_tile_active(s)) launch_slopes(s, which);  // the tile kernel computes slopes itself
   }
-  else if (s->desc.reconstruction == H3C_RECON_MUSCL) launch_grad(s, q);
+  else if (s->desc.reconstruction == H3C_RECON_MUSCL) launch_grad(s, q, false);
 }
 
 // One solver step (solver.hpp:140-145) on the solver's buffers.  keep (may be
@@ -1417,26 +1440,63 @@ static int stage_count(const h3c_solver s) {
   return ti == H3C_EULER_FORWARD ? 1 : ti == H3C_RUNGE_KUTTA_2 ? 2 : 3;
 }
 
+// The ghosts no condition writes (hom3's segments can leave some out, and
+// exchange ghosts are the caller's) keep the start state's values in the third
+// SSP-RK3 buffer.
+static void copy_loose_ghosts(h3c_solver s, double* dst, const double* src) {
+  if (!s->ghost_unapplied && !s->has_exchange) return;
+  cudaMemcpy2DAsync(dst + s->n_int, sizeof(double) * s->ld, src + s->n_int, sizeof(double) * s->ld,
+                    sizeof(double) * s->ng, s->nv, cudaMemcpyDeviceToDevice, s->stream);
+}
+
 // Part k of one step (k = 0 .. stage_count - 1, in order): k = 0 applies the
 // conditions to lhs and sets the step's dt; k > 0 applies the conditions to
 // its stage input; every part then runs its stage; the last part advances
 // time and step.  keep (optional) receives each stage's input; dts (optional)
-// records the step's dt at index i.
-static void enqueue_stage(h3c_solver s, int k, bool fuse, double* keep, double* dts, long long i) {
+// records the step's dt at index i.  whole: all parts follow at once, so the
+// kernel of the first conditions also sets dt and advances (StepBegin; not
+// with a condition that rewrites interior cells, whose dt needs them first
+// and which reads the time).  heat: the coupled loop's second solver, whose
+// scalars are set with this one's.
+struct Coupled {
+  h3c_solver heat = nullptr;
+  double scaling = 1.0;
+  double* dts = nullptr;
+};
+static void enqueue_stage(h3c_solver s, int k, bool fuse, bool whole, double* keep, double* dts, long long i,
+                          const Coupled* cpl = nullptr, bool begun = false) {
   const size_t Qb = sizeof(double) * s->nv * s->ld;
   const long long Q = s->nv * s->ld;
   const int ti = s->desc.time_integration;
   const int last = stage_count(s) - 1;
+  whole = whole && fuse;
   if (k == 0) {
-    launch_bc(s, 0);
-    if (!fuse) launch_cfl(s, &s->d_sc->dtmin_ord);
-    {
-      Launch L(s, K_SCALAR);
-      k_set_dt<<<blocks(s->n_inst), kBlock, 0, s->stream>>>(s->d_sc, 1, s->n_inst);
-    }
-    if (dts) {
-      Launch L(s, K_SCALAR);
-      k_record_dt<<<1, 1, 0, s->stream>>>(s->d_sc, dts, i);
+    if (begun) {  // the coupled loop's first solver has set this one's scalars
+      launch_bc(s, 0);
+    } else if (whole) {
+      StepBegin b;
+      b.sc = s->d_sc;
+      b.n_inst = s->n_inst;
+      b.advance = 1;
+      b.record = dts;
+      b.idx = i;
+      if (cpl) {
+        b.heat = cpl->heat->d_sc;
+        b.scaling = cpl->scaling;
+        b.heat_record = cpl->dts;
+      }
+      launch_bc_ptr(s, s->d_q[0], s->d_q[0], b);
+    } else {
+      launch_bc(s, 0);
+      if (!fuse) launch_cfl(s, &s->d_sc->dtmin_ord);
+      {
+        Launch L(s, K_SCALAR);
+        k_set_dt<<<blocks(s->n_inst), kBlock, 0, s->stream>>>(s->d_sc, 1, s->n_inst);
+      }
+      if (dts) {
+        Launch L(s, K_SCALAR);
+        k_record_dt<<<1, 1, 0, s->stream>>>(s->d_sc, dts, i);
+      }
     }
     if (keep) cudaMemcpyAsync(keep, s->d_q[0], Qb, cudaMemcpyDeviceToDevice, s->stream);
     prepare_stage(s, s->d_q[0], 0);
@@ -1451,14 +1511,13 @@ static void enqueue_stage(h3c_solver s, int k, bool fuse, double* keep, double* 
   } else if (k == 1) {
     launch_bc(s, 1);
     if (keep) cudaMemcpyAsync(keep + Q, s->d_q[1], Qb, cudaMemcpyDeviceToDevice, s->stream);
+    prepare_stage(s, s->d_q[1], 1);
+    // EXTENSION: SSP-RK3, conditions before every stage
     if (ti == H3C_RUNGE_KUTTA_2) {
-      prepare_stage(s, s->d_q[1], 1);
       launch_stage(s, 2, s->d_q[1], s->d_q[0], fuse);
     } else {
-      // EXTENSION: SSP-RK3, conditions before every stage
-      cudaMemcpyAsync(s->d_q[2], s->d_q[0], Qb, cudaMemcpyDeviceToDevice, s->stream);
-      prepare_stage(s, s->d_q[1], 1);
-      launch_stage(s, 3, s->d_q[1], s->d_q[2], false);
+      copy_loose_ghosts(s, s->d_q[2], s->d_q[0]);
+      launch_stage(s, 3, s->d_q[1], s->d_q[2], false, s->d_q[0]);
     }
   } else {
     launch_bc(s, 2);
@@ -1466,14 +1525,15 @@ static void enqueue_stage(h3c_solver s, int k, bool fuse, double* keep, double* 
     prepare_stage(s, s->d_q[2], 2);
     launch_stage(s, 4, s->d_q[2], s->d_q[0], fuse);
   }
-  if (k == last) {
+  if (k == last && !whole && !begun) {
     Launch L(s, K_SCALAR);
     k_advance<<<blocks(s->n_inst), kBlock, 0, s->stream>>>(s->d_sc, s->n_inst);
   }
 }
 
-static void enqueue_step(h3c_solver s, bool fuse, double* keep, double* dts, long long i) {
-  for (int k = 0; k < stage_count(s); ++k) enqueue_stage(s, k, fuse, keep, dts, i);
+static void enqueue_step(h3c_solver s, bool fuse, double* keep, double* dts, long long i, const Coupled* cpl = nullptr,
+                         bool begun = false) {
+  for (int k = 0; k < stage_count(s); ++k) enqueue_stage(s, k, fuse, true, keep, dts, i, cpl, begun);
 }
 
 static void enqueue_steps(h3c_solver s, int64_t nsteps) {
@@ -1561,6 +1621,7 @@ int h3c_solve(h3c_solver s, int64_t nsteps) {
   // run plainly (kernel attributes are set outside capture); coupled solvers
   // read their partner's current buffers and profiling brackets every
   // launch, so those take the plain path.
+  const int64_t total = nsteps;
   const bool graphable = s->graphs && !s->prof && s->partner == nullptr;
   if (graphable && !s->plain_done && nsteps > 0) {
     enqueue_steps(s, 1);
@@ -1578,6 +1639,7 @@ int h3c_solve(h3c_solver s, int64_t nsteps) {
     enqueue_steps(s, nsteps);
     s->plain_done = true;
   }
+  if (total > 0) s->mirror_valid = s->h_mirror && !s->unfused_dt;
   return s->cuda(cudaGetLastError(), "h3c_solve");
 }
 
@@ -1594,7 +1656,8 @@ int h3c_solve_stage(h3c_solver s, int k) {
   if (int rc = ready(s, "h3c_solve_stage")) return rc;
   if (k != s->stage_next)
     return s->fail(H3C_E_STATE, "h3c_solve_stage: part %d requested, part %d is next", k, s->stage_next);
-  enqueue_stage(s, k, !s->unfused_dt, nullptr, nullptr, 0);
+  s->mirror_valid = false;
+  enqueue_stage(s, k, !s->unfused_dt, false, nullptr, nullptr, 0);
   s->stage_next = k + 1 == stage_count(s) ? 0 : k + 1;
   return s->cuda(cudaGetLastError(), "h3c_solve_stage");
 }
@@ -1614,7 +1677,18 @@ int h3c_dtmin_device(h3c_solver s, int64_t** ptr) {
   return H3C_OK;
 }
 
-static int read_scalars(h3c_solver s, Scalars* out) {
+// dt, time, step and status of instance 0 after the work enqueued so far: from
+// the mirror where the last step wrote it, else copied from the device.
+static int read_scalars(h3c_solver s, Scalars* out, bool mirrored = false) {
+  if (mirrored && s->mirror_valid) {
+    H3C_CUDA(s, cudaStreamSynchronize(s->stream));
+    const volatile HostScalars* m = s->h_mirror;
+    out->dt = m->dt;
+    out->time = m->time;
+    out->step = m->step;
+    out->status = m->status | (m->bad_state ? kStatusState : 0) | (m->timeout ? kStatusTimeout : 0);
+    return H3C_OK;
+  }
   Scalars* dst = s->h_sc ? s->h_sc : out;
   H3C_CUDA(s, cudaMemcpyAsync(dst, s->d_sc, sizeof(Scalars), cudaMemcpyDeviceToHost, s->stream));
   H3C_CUDA(s, cudaStreamSynchronize(s->stream));
@@ -1663,7 +1737,7 @@ int h3c_min_dt(h3c_solver s, double* dt) {
 int h3c_dt(h3c_solver s, double* dt) {
   if (!s || !dt) return H3C_E_INVALID;
   Scalars sc;
-  int rc = read_scalars(s, &sc);
+  int rc = read_scalars(s, &sc, true);
   if (rc) return rc;
   *dt = sc.dt;
   return status_error(s, sc);
@@ -1671,7 +1745,7 @@ int h3c_dt(h3c_solver s, double* dt) {
 int h3c_time(h3c_solver s, double* t) {
   if (!s || !t) return H3C_E_INVALID;
   Scalars sc;
-  int rc = read_scalars(s, &sc);
+  int rc = read_scalars(s, &sc, true);
   if (rc) return rc;
   *t = sc.time;
   return status_error(s, sc);
@@ -1679,7 +1753,7 @@ int h3c_time(h3c_solver s, double* t) {
 int h3c_step(h3c_solver s, int64_t* step) {
   if (!s || !step) return H3C_E_INVALID;
   Scalars sc;
-  int rc = read_scalars(s, &sc);
+  int rc = read_scalars(s, &sc, true);
   if (rc) return rc;
   *step = sc.step;
   return status_error(s, sc);
@@ -1687,12 +1761,14 @@ int h3c_step(h3c_solver s, int64_t* step) {
 int h3c_force_dt(h3c_solver s, double dt) {
   if (!s) return H3C_E_INVALID;
   if (!s->has_grid) return s->fail(H3C_E_STATE, "h3c_force_dt: no grid");
+  s->mirror_valid = false;
   k_force_dt<<<1, 1, 0, s->stream>>>(s->d_sc, dt);
   return s->cuda(cudaGetLastError(), "h3c_force_dt");
 }
 int h3c_status(h3c_solver s, int* flags) {
   if (!s || !flags) return H3C_E_INVALID;
   if (!s->has_grid) return s->fail(H3C_E_STATE, "h3c_status: no grid");
+  s->mirror_valid = false;
   std::vector<Scalars> h(s->n_inst);
   H3C_CUDA(s, cudaMemcpyAsync(h.data(), s->d_sc, sizeof(Scalars) * s->n_inst, cudaMemcpyDeviceToHost, s->stream));
   H3C_CUDA(s, cudaStreamSynchronize(s->stream));
@@ -1761,8 +1837,16 @@ int h3c_set_periodic(h3c_solver s, const int64_t* partner_cells) {
       return s->fail(H3C_E_INVALID, "h3c_set_periodic: periodic ghost %lld has no interior partner", i);
   }
   H3C_CUDA(s, cudaMemcpy(s->d_gpartner, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice));
+  if (s->desc.reconstruction == H3C_RECON_MUSCL) {
+    std::vector<int> src(h.size());
+    for (long long i = 0; i < (long long)h.size(); ++i)
+      src[i] = i < s->ng && s->h_bcs[own[i]].kind == H3C_BC_PERIODIC ? h[i] : (int)(s->n_int + i);
+    if (!s->d_gsrc) H3C_CUDA(s, cudaMalloc(&s->d_gsrc, sizeof(int) * src.size()));
+    H3C_CUDA(s, cudaMemcpy(s->d_gsrc, src.data(), sizeof(int) * src.size(), cudaMemcpyHostToDevice));
+  }
   H3C_CUDA(s, cudaStreamSynchronize(cudaStreamLegacy));  // the copy lands before the stream's kernels read it
   s->periodic_set = true;
+  drop_graph(s);
   return H3C_OK;
 }
 
@@ -1779,19 +1863,36 @@ int h3c_couple_cht(h3c_solver cns, h3c_solver heat, double Tr0) {
   return cns->cuda(cudaGetLastError(), "h3c_couple_cht");
 }
 
-// One coupled step: coupling::apply(Tr0, cns, heat), cns.solve(), heat.solve()
-// (coupled_cns_heat_test.cpp:235-248), all on the shared stream.
-static void enqueue_cht(h3c_solver cns, h3c_solver heat, double scaling, int64_t n) {
+// n coupled steps: coupling::apply(Tr0, cns, heat), cns.solve(), heat.solve()
+// (coupled_cns_heat_test.cpp:235-248), all on the shared stream.  The kernel
+// that applies the fluid's conditions takes both solvers' minima -- the fused
+// reductions of their last stages (coupled_begin refreshes them) -- and sets
+// both time steps: five launches a step where the three calls make fourteen.
+// dtf, dth (optional): record the time steps at [0, n).
+static void enqueue_cht(h3c_solver cns, h3c_solver heat, double scaling, int64_t n, double* dtf = nullptr,
+                        double* dth = nullptr) {
+  const bool fused = !cns->unfused_dt && !heat->unfused_dt;
   for (int64_t i = 0; i < n; ++i) {
+    if (fused) {
+      const Coupled cpl{heat, scaling, dth};
+      enqueue_step(cns, true, nullptr, dtf, i, &cpl);
+      enqueue_step(heat, true, nullptr, nullptr, 0, nullptr, true);
+      continue;
+    }
     launch_cfl(cns, &cns->d_sc->mindt_ord);
     launch_cfl(heat, &heat->d_sc->mindt_ord);
     {
       Launch L(cns, K_SCALAR);
       k_couple_cht<<<1, 1, 0, cns->stream>>>(cns->d_sc, heat->d_sc, scaling);
     }
-    enqueue_steps(cns, 1);
-    enqueue_steps(heat, 1);
+    enqueue_step(cns, !cns->unfused_dt, nullptr, dtf, i);
+    enqueue_step(heat, !heat->unfused_dt, nullptr, dth, i);
   }
+}
+// before the first of a run of coupled steps: the minima of the states as they are now
+static void coupled_begin(h3c_solver cns, h3c_solver heat) {
+  launch_cfl(cns, &cns->d_sc->dtmin_ord);
+  launch_cfl(heat, &heat->d_sc->dtmin_ord);
 }
 
 int h3c_cht_solve(h3c_solver cns, h3c_solver heat, double Tr0, int64_t nsteps) {
@@ -1803,7 +1904,9 @@ int h3c_cht_solve(h3c_solver cns, h3c_solver heat, double Tr0, int64_t nsteps) {
     return cns->fail(H3C_E_INVALID, "h3c_cht_solve: expects (cns, heat)");
   if (cns->stream != heat->stream || cns->partner != heat || heat->partner != cns)
     return cns->fail(H3C_E_STATE, "h3c_cht_solve: solvers are not coupled with each other");
+  if (nsteps == 0) return H3C_OK;
   const double scaling = Tr0 * cns->Pr0 * cns->Re0;
+  coupled_begin(cns, heat);
   const bool graphable = cns->graphs && heat->graphs && !cns->prof && !heat->prof;
   if (graphable && nsteps >= kGraphSteps) {
     if (cns->cpl_graph && (cns->cpl_with != heat || cns->cpl_q0 != cns->d_q[0] ||
@@ -1839,6 +1942,7 @@ int h3c_cht_solve(h3c_solver cns, h3c_solver heat, double Tr0, int64_t nsteps) {
     }
   }
   enqueue_cht(cns, heat, scaling, nsteps);
+  for (h3c_solver x : {cns, heat}) x->mirror_valid = x->h_mirror && !cns->unfused_dt && !heat->unfused_dt;
   return cns->cuda(cudaGetLastError(), "h3c_cht_solve");
 }
 
@@ -2002,6 +2106,7 @@ int h3c_autotune(h3c_solver s, int nsteps, int* choice, double* ms_out) {
   cudaMemcpyAsync(save + s->nv * s->ld, q1, qbytes, cudaMemcpyDeviceToDevice, s->stream);
   cudaMemcpyAsync(save_sc, s->d_sc, sizeof(Scalars) * s->n_inst, cudaMemcpyDeviceToDevice, s->stream);
   auto restore = [&]() {
+    s->mirror_valid = false;
     s->d_q[0] = q0;  // forward Euler swaps the buffers
     s->d_q[1] = q1;
     cudaMemcpyAsync(q0, save, qbytes, cudaMemcpyDeviceToDevice, s->stream);
@@ -2074,43 +2179,46 @@ static int adjoint_supported(h3c_solver s, const char* what, bool coupled = fals
 
 // One step with the given time step on explicit buffers.  st[0] is the
 // step's start state; the stage inputs (ghosts filled) are left in st[0..]
-// (RK2: st[1]; SSP-RK3: st[1], st[2]) and the new state in out.  For forward
-// Euler out must not alias st[0]; for the Runge-Kutta schemes out == st[0] is
-// allowed (in-place last stage), otherwise st[0] is copied to out first.
+// (RK2: st[1]; SSP-RK3: st[1], st[2]) and the new state's interior cells in
+// out.  For forward Euler out must not alias st[0]; for the Runge-Kutta
+// schemes out == st[0] is allowed (in-place last stage).
 static void frozen_step(h3c_solver s, double* const* st, double* out, const double* d_dts, long long i) {
-  const size_t Qb = sizeof(double) * s->nv * s->ld;
-  launch_bc_ptr(s, st[0], st[0]);
-  {
+  const int ti = s->desc.time_integration;
+  const bool cns = s->desc.physics == H3C_CNS, muscl = s->desc.reconstruction == H3C_RECON_MUSCL;
+  auto prepare = [&](const double* q) {
+    if (muscl) launch_grad(s, q, false);
+    if (cns && !cns_tile_active(s)) launch_slopes_ptr(s, q);
+  };
+  if (s->unfused_dt) {  // the vortex condition reads the time: scalars apart, in hom3's order
+    launch_bc_ptr(s, st[0], st[0]);
     Launch L(s, K_SCALAR);
     k_set_dt_from<<<1, 1, 0, s->stream>>>(s->d_sc, d_dts, i);
+  } else {
+    StepBegin b;
+    b.sc = s->d_sc;
+    b.advance = 1;
+    b.from = d_dts;
+    b.idx = i;
+    launch_bc_ptr(s, st[0], st[0], b);
   }
-  const int ti = s->desc.time_integration;
-  const bool cns = s->desc.physics == H3C_CNS;
-  if (s->desc.reconstruction == H3C_RECON_MUSCL) launch_grad(s, st[0]);
-  if (cns) launch_slopes_ptr(s, st[0]);
+  prepare(st[0]);
   if (ti == H3C_EULER_FORWARD) {
     launch_stage(s, 0, st[0], out, false);
-  } else if (ti == H3C_RUNGE_KUTTA_2) {
-    launch_stage(s, 0, st[0], st[1], false);
-    launch_bc_ptr(s, st[1], st[0]);
-    if (out != st[0]) cudaMemcpyAsync(out, st[0], Qb, cudaMemcpyDeviceToDevice, s->stream);
-    if (s->desc.reconstruction == H3C_RECON_MUSCL) launch_grad(s, st[1]);
-    if (cns) launch_slopes_ptr(s, st[1]);
-    launch_stage(s, 2, st[1], out, false);
   } else {
     launch_stage(s, 0, st[0], st[1], false);
     launch_bc_ptr(s, st[1], st[0]);
-    cudaMemcpyAsync(st[2], st[0], Qb, cudaMemcpyDeviceToDevice, s->stream);
-    if (s->desc.reconstruction == H3C_RECON_MUSCL) launch_grad(s, st[1]);
-    if (cns) launch_slopes_ptr(s, st[1]);
-    launch_stage(s, 3, st[1], st[2], false);
-    launch_bc_ptr(s, st[2], st[0]);
-    if (out != st[0]) cudaMemcpyAsync(out, st[0], Qb, cudaMemcpyDeviceToDevice, s->stream);
-    if (s->desc.reconstruction == H3C_RECON_MUSCL) launch_grad(s, st[2]);
-    if (cns) launch_slopes_ptr(s, st[2]);
-    launch_stage(s, 4, st[2], out, false);
+    prepare(st[1]);
+    if (ti == H3C_RUNGE_KUTTA_2) {
+      launch_stage(s, 2, st[1], out, false, st[0]);
+    } else {
+      copy_loose_ghosts(s, st[2], st[0]);
+      launch_stage(s, 3, st[1], st[2], false, st[0]);
+      launch_bc_ptr(s, st[2], st[0]);
+      prepare(st[2]);
+      launch_stage(s, 4, st[2], out, false, st[0]);
+    }
   }
-  {
+  if (s->unfused_dt) {
     Launch L(s, K_SCALAR);
     k_advance<<<1, 1, 0, s->stream>>>(s->d_sc, 1);
   }
@@ -2122,6 +2230,7 @@ int h3c_solve_dt(h3c_solver s, int64_t nsteps, const double* dts) {
   if (int rc = ready(s, "h3c_solve_dt")) return rc;
   if (s->n_inst != 1) return s->fail(H3C_E_INVALID, "h3c_solve_dt: single grids only");
   if (nsteps == 0) return H3C_OK;
+  s->mirror_valid = false;
   double* d_dts = nullptr;
   H3C_CUDA(s, cudaMalloc(&d_dts, sizeof(double) * nsteps));
   cudaMemcpyAsync(d_dts, dts, sizeof(double) * nsteps, cudaMemcpyHostToDevice, s->stream);
@@ -2149,6 +2258,7 @@ int h3c_adjoint(h3c_solver s, int64_t nsteps, int64_t every, const double* dJ_dq
   Range r("h3c_adjoint");
   if (!s || nsteps < 1 || every < 0 || !dJ_dqN || !dJ_dq0) return H3C_E_INVALID;
   if (int rc = adjoint_supported(s, "h3c_adjoint")) return rc;
+  s->mirror_valid = false;
   const long long L = s->ld, nv = s->nv, Q = nv * L;
   const int ti = s->desc.time_integration;
   const long long per = ti == H3C_EULER_FORWARD ? 1 : ti == H3C_RUNGE_KUTTA_2 ? 2 : 3;  // stages per step
@@ -2243,7 +2353,7 @@ int h3c_adjoint(h3c_solver s, int64_t nsteps, int64_t every, const double* dJ_dq
       return;
     }
     if (muscl) {
-      launch_grad(s, qin);  // the forward's limited gradients of this stage input
+      launch_grad(s, qin, true);  // the forward's limited gradients of this stage input
       Launch La(s, K_OTHER);
       const unsigned nb = (unsigned)blocks(s->n_int);
       const double K = s->desc.limiter_k;
@@ -2412,6 +2522,7 @@ int h3c_cht_adjoint(h3c_solver cns, h3c_solver heat, double Tr0, int64_t nsteps,
   if (cns->desc.time_integration != H3C_EULER_FORWARD || heat->desc.time_integration != H3C_EULER_FORWARD)
     return cns->fail(H3C_E_INVALID, "h3c_cht_adjoint: forward Euler (the coupled loop's scheme) only");
   if (cns->unfused_dt || heat->unfused_dt) return cns->fail(H3C_E_INVALID, "h3c_cht_adjoint: unsupported condition");
+  cns->mirror_valid = heat->mirror_valid = false;
   if (every == 0 || every > nsteps) every = std::min<int64_t>(nsteps, every == 0 ? 100 : every);
   const double scaling = Tr0 * cns->Pr0 * cns->Re0;
   const long long Qf = (long long)cns->nv * cns->ld, Qs = (long long)heat->nv * heat->ld;
@@ -2478,18 +2589,8 @@ int h3c_cht_adjoint(h3c_solver cns, h3c_solver heat, double Tr0, int64_t nsteps,
   if (int rc = ensure_stage(cns, cns->n_caller)) { cudaFree(ws); return rc; }
   if (int rc = ensure_stage(heat, heat->n_caller)) { cudaFree(ws); return rc; }
   // ---- forward: the coupled loop (coupling::apply, cns step, heat step), checkpoints, dt records ----
-  auto fwd_seg = [&](long long n) {
-    for (long long j = 0; j < n; ++j) {
-      launch_cfl(cns, &cns->d_sc->mindt_ord);
-      launch_cfl(heat, &heat->d_sc->mindt_ord);
-      {
-        Launch L(cns, K_SCALAR);
-        k_couple_cht<<<1, 1, 0, st>>>(cns->d_sc, heat->d_sc, scaling);
-      }
-      enqueue_step(cns, true, nullptr, sdtf, j);
-      enqueue_step(heat, true, nullptr, sdth, j);
-    }
-  };
+  auto fwd_seg = [&](long long n) { enqueue_cht(cns, heat, scaling, n, sdtf, sdth); };
+  coupled_begin(cns, heat);
   for (long long k = 0; k < nck; ++k) {
     const long long i0 = k * every, i1 = std::min<long long>(nsteps, i0 + every);
     cudaMemcpyAsync(ckf + Qf * k, cns->d_q[0], sizeof(double) * Qf, cudaMemcpyDeviceToDevice, st);

@@ -33,6 +33,7 @@
 #include "fv_kernels.cuh"
 #include "stage_halo.hpp"
 #include "async_copy.cuh"
+#include "launch.hpp"
 
 namespace h3c {
 
@@ -44,6 +45,7 @@ template <int ND>
 __global__ void __launch_bounds__(kBlock) k_ghost_slopes(const double* __restrict__ q, Geometry g, GhostTables gt,
                                                          double* __restrict__ gsl, long long ngl) {
   constexpr int NV = ND + 2;
+  chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= gt.ng) return;
   const long long ld = g.ld;
@@ -125,6 +127,7 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
     return land + (size_t)v * S + s;
   };
 
+  chain_begin();
   long long tile = blockIdx.x;
   if (tile >= g.ntiles) return;
   if (tid == 0) {
@@ -229,12 +232,12 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
     const int inst = tile_instance(g, tile);
     const long long te = min(c0 + (long long)TB, instance_end(g, inst));
     const bool live = c < te;
-    if (MODE != 0 && live) prefetch_row_l2<NV>(out, ld, c);  // the in-place start state, read at the update
+    if (MODE != 0 && live) prefetch_row_l2<NV>(g.q0, ld, c);  // the start state, read at the update
 
     const bool ok = mbar_wait_bounded(bar, (unsigned)(it & 1));
     cp_async_wait_all();
     if (!__syncthreads_and(ok)) {
-      if (tid == 0) atomicOr(status, kStatusTimeout);
+      if (tid == 0) flag_timeout(sc, status);
       return;
     }
 
@@ -340,7 +343,7 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
       for (int v = 0; v < NV; ++v) qc[v] = LIP ? *qslot(v, tid) : __ldg(qin + v * ld + c);
       if (MODE != 0) {
 #pragma unroll
-        for (int v = 0; v < NV; ++v) qo[v] = out[v * ld + c];
+        for (int v = 0; v < NV; ++v) qo[v] = g.q0[v * ld + c];
       }
       double o[NV];
 #pragma unroll
@@ -530,8 +533,12 @@ template <int ND, class R, int MODE>
 void claunch_f(bool fuse, const double* qin, double* out, const Geometry& g, const CnsHaloGeom& h,
                const PhysConst& pc, const Scalars* sc, long long* dtmin, int* status, int grid, size_t smem,
                cudaStream_t st) {
-  if (fuse) k_stage_cns_halo<ND, R, MODE, true><<<grid, kHaloTile, smem, st>>>(qin, out, g, h, pc, sc, dtmin, status);
-  else k_stage_cns_halo<ND, R, MODE, false><<<grid, kHaloTile, smem, st>>>(qin, out, g, h, pc, sc, dtmin, status);
+  const auto k = fuse ? k_stage_cns_halo<ND, R, MODE, true> : k_stage_cns_halo<ND, R, MODE, false>;
+  // Chained (launch.hpp) where blocks take few tiles: 64^3 FP32 1141 -> 1106 us per 10 steps.  On long runs of
+  // tiles per block the early start is worth nothing, and blocks that find an SM still taken by the kernel
+  // before finish last (128^3, 28 tiles per block: 3205 -> 3245 us per 4 steps).
+  if (g.ntiles <= 8LL * grid) launch_chain(k, grid, kHaloTile, smem, st, qin, out, g, h, pc, sc, dtmin, status);
+  else k<<<grid, kHaloTile, smem, st>>>(qin, out, g, h, pc, sc, dtmin, status);
 }
 template <int ND, class R>
 void claunch_m(int mode, bool fuse, const double* qin, double* out, const Geometry& g, const CnsHaloGeom& h,
@@ -557,8 +564,7 @@ void cns_halo_stage(int nd, bool mixed, int mode, bool fuse, const double* qin, 
                     long long* dtmin, int* status, int grid, size_t smem, cudaStream_t st, double* gsl) {
   if (gt.ng > 0) {
     const unsigned nb = (unsigned)((gt.ng + kBlock - 1) / kBlock);
-    if (nd == 2) k_ghost_slopes<2><<<nb, kBlock, 0, st>>>(qin, g, gt, gsl, h.ngl);
-    else k_ghost_slopes<3><<<nb, kBlock, 0, st>>>(qin, g, gt, gsl, h.ngl);
+    launch_chain(nd == 2 ? k_ghost_slopes<2> : k_ghost_slopes<3>, nb, kBlock, 0, st, qin, g, gt, gsl, h.ngl);
   }
   if (nd == 2) {
     if (mixed) claunch_m<2, float>(mode, fuse, qin, out, g, h, pc, sc, dtmin, status, grid, smem, st);

@@ -161,14 +161,14 @@ __global__ void __launch_bounds__(kHaloTile, 3)
     double qo[NV];
     if (MODE != 0 && live) {
 #pragma unroll
-      for (int v = 0; v < NV; ++v) qo[v] = out[v * ld + c];
+      for (int v = 0; v < NV; ++v) qo[v] = g.q0[v * ld + c];
     }
 
     // ---- this tile's copies ----
     const bool ok = mbar_wait_bounded(bar, (unsigned)(it & 1));
     cp_async_wait_all();
     if (!__syncthreads_and(ok)) {
-      if (tid == 0) atomicOr(status, kStatusTimeout);
+      if (tid == 0) flag_timeout(sc, status);
       return;
     }
 

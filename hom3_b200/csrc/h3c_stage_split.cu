@@ -39,6 +39,7 @@
 #define H3C_DEVICE_FUNCTIONS_ONLY
 #include "fv_kernels.cuh"
 #include "stage_split.hpp"
+#include "launch.hpp"
 #include "async_copy.cuh"
 
 namespace h3c {
@@ -122,6 +123,7 @@ __global__ void __launch_bounds__(kHaloTile, split_minb<ND, R>())
   const int tid = threadIdx.x;
   const long long ld = g.ld;
   const R gamma = (R)pc.gamma, gm1 = (R)pc.gm1;
+  chain_begin();
 
   // theta of the state in P.q into slot s; P keeps p, a and the Mach numbers
   auto store_theta = [&](int s, Prim<R, ND>& P) {
@@ -180,9 +182,9 @@ __global__ void __launch_bounds__(kHaloTile, split_minb<ND, R>())
     if (live) {
       if (ND == 3) asm volatile("prefetch.global.L2 [%0];" ::"l"(sg.pack3 + c));
       else asm volatile("prefetch.global.L2 [%0];" ::"l"(sg.pack2 + c));
-      if (MODE != 0) {  // the in-place start state, read at the update
+      if (MODE != 0) {  // the start state, read at the update
 #pragma unroll
-        for (int v = 0; v < NV; ++v) asm volatile("prefetch.global.L2 [%0];" ::"l"(at32(out + v * ld, c)));
+        for (int v = 0; v < NV; ++v) asm volatile("prefetch.global.L2 [%0];" ::"l"(at32(g.q0 + v * ld, c)));
       }
     }
     if (tid < kMaxLevels) skdt[tid] = sc[inst].dt / g.len[tid];
@@ -398,7 +400,7 @@ __global__ void __launch_bounds__(kHaloTile, split_minb<ND, R>())
       double qo[NV];
       if (MODE != 0) {
 #pragma unroll
-        for (int v = 0; v < NV; ++v) qo[v] = *at32(out + v * ld, c);
+        for (int v = 0; v < NV; ++v) qo[v] = *at32(g.q0 + v * ld, c);
       }
       const double k = skdt[lev];
       double o[NV];
@@ -490,8 +492,8 @@ struct SplitLaunch {
 };
 template <int ND, class R, int MODE, bool HANG>
 void slaunch_f(bool fuse, const SplitLaunch& a) {
-  if (fuse) k_stage_split<ND, R, MODE, HANG, true><<<a.grid, kHaloTile, a.smem, a.st>>>(a.qin, a.out, a.g, a.h, a.pc, a.sc, a.dtmin);
-  else k_stage_split<ND, R, MODE, HANG, false><<<a.grid, kHaloTile, a.smem, a.st>>>(a.qin, a.out, a.g, a.h, a.pc, a.sc, a.dtmin);
+  launch_chain(fuse ? k_stage_split<ND, R, MODE, HANG, true> : k_stage_split<ND, R, MODE, HANG, false>, a.grid,
+               kHaloTile, a.smem, a.st, a.qin, a.out, a.g, a.h, a.pc, a.sc, a.dtmin);
 }
 template <int ND, class R, int MODE>
 void slaunch_h(bool hang, bool fuse, const SplitLaunch& a) {

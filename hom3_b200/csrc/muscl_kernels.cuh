@@ -11,7 +11,8 @@
 //    phi(a, b) = ((a^2 + e) b + 2 b^2 a) / (b (a^2 + 2 b^2 + a b + e)),
 //    e = (K h)^3.  Stores psi_v G_v.
 //  * k_muscl_ghosts: periodic ghosts take their paired cell's gradient; other
-//    ghosts keep a zero gradient (first order on the ghost side).
+//    ghosts keep a zero gradient (first order on the ghost side).  The stage
+//    itself reads the paired cell's (gsrc), so only the adjoint runs this.
 //  * k_stage_muscl: per cell, every face evaluates AUSM on the reconstructed
 //    states w + psi G . (x_f - x) of both sides at one face point (on the face
 //    plane, transverse coordinates of the smaller cell), falling back to the
@@ -77,6 +78,7 @@ __global__ void __launch_bounds__(kBlock) k_muscl_grad(const double* __restrict_
                                                        Geometry g, PhysConst pc, double limiter_k,
                                                        double* __restrict__ grad) {
   constexpr int NV = ND + 2;
+  chain_begin();
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= instance_end(g, tile_instance(g, blockIdx.x))) return;  // also skips padding between instances
   const long long ld = g.ld;
@@ -226,8 +228,10 @@ template <int ND, class R, int MODE, bool HANG, bool FUSE>
 __global__ void __launch_bounds__(kBlock) k_stage_muscl(const double* __restrict__ qin, double* out,
                                                         const double* __restrict__ grad,
                                                         const double* __restrict__ xc, Geometry g, PhysConst pc,
-                                                        const Scalars* __restrict__ sc, long long* dtmin) {
+                                                        const Scalars* __restrict__ sc, long long* dtmin,
+                                                        const int* __restrict__ gsrc) {
   constexpr int NV = ND + 2;
+  chain_begin();
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int inst = tile_instance(g, blockIdx.x);
   const bool live = c < instance_end(g, inst);
@@ -255,6 +259,8 @@ __global__ void __launch_bounds__(kBlock) k_stage_muscl(const double* __restrict
       const int L = side < 0 ? n : (int)c, Rr = side < 0 ? (int)c : n;
       double xf[ND];
       face_point<ND>(g, xc, L, Rr, d, xf);
+      // a periodic ghost's gradient is its paired cell's (gsrc; the others' are zero where they are stored)
+      const int gn = gsrc && n >= g.n_int ? __ldg(gsrc + (n - g.n_int)) : n;
       double wn[NV], xn[ND];
       prim_w<ND>(qin, ld, n, gm1, wn);
 #pragma unroll
@@ -268,7 +274,7 @@ __global__ void __launch_bounds__(kBlock) k_stage_muscl(const double* __restrict
         wcf[v] = s;
         double t = wn[v];
 #pragma unroll
-        for (int k = 0; k < ND; ++k) t = t + __ldg(grad + (v * ND + k) * ld + n) * (xf[k] - xn[k]);
+        for (int k = 0; k < ND; ++k) t = t + __ldg(grad + (v * ND + k) * ld + gn) * (xf[k] - xn[k]);
         wnf[v] = t;
       }
       if (!(wcf[ND] > 0) || !(wcf[ND + 1] > 0) || !(wnf[ND] > 0) || !(wnf[ND + 1] > 0)) {
@@ -312,7 +318,7 @@ __global__ void __launch_bounds__(kBlock) k_stage_muscl(const double* __restrict
     const double k = dt / dx;
     double o[NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) o[v] = rk_combine<MODE>(MODE == 0 ? 0.0 : out[v * ld + c], qc[v], k * acc[v]);
+    for (int v = 0; v < NV; ++v) o[v] = rk_combine<MODE>(MODE == 0 ? 0.0 : g.q0[v * ld + c], qc[v], k * acc[v]);
 #pragma unroll
     for (int v = 0; v < NV; ++v) out[v * ld + c] = o[v];
     if (FUSE) {

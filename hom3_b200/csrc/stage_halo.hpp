@@ -74,7 +74,7 @@ int halo_slots_for(int nd, bool mixed, int max_halo, int blocks_per_sm);
 // the kernel cannot be launched with it).  Call outside stream capture.
 int halo_prepare(int nd, bool mixed, size_t smem);
 
-// One stage: out = rk_combine<mode>(out, qin, dt/dx R(qin)) over the tiles,
+// One stage: out = rk_combine<mode>(g.q0, qin, dt/dx R(qin)) over the tiles,
 // with the fused next-step CFL minimum into dtmin when fuse.  grid blocks
 // take the tiles round-robin.  status receives bit 2 when a bounded wait for
 // a tile's copies runs out.

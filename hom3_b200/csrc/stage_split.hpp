@@ -24,7 +24,7 @@ size_t split_smem_bytes(int nd, bool mixed);
 // (outside capture); false when the kernel cannot be launched.
 bool split_prepare(int nd, bool mixed, size_t smem);
 
-// One stage: out = rk_combine<mode>(out, qin, dt/dx R(qin)), with the fused
+// One stage: out = rk_combine<mode>(g.q0, qin, dt/dx R(qin)), with the fused
 // next-step CFL minimum into dtmin when fuse; grid blocks take the tiles round-robin.
 void split_stage(int nd, bool mixed, int mode, bool hang, bool fuse, const double* qin, double* out,
                  const Geometry& g, const SplitGeom& h, const PhysConst& pc, const Scalars* sc, long long* dtmin,

@@ -29,7 +29,7 @@ size_t warp_smem_bytes(int nd, bool mixed);
 // outside stream capture.
 int warp_prepare(int nd, bool mixed);
 
-// One stage: out = rk_combine<mode>(out, qin, dt/dx R(qin)) over the interior
+// One stage: out = rk_combine<mode>(g.q0, qin, dt/dx R(qin)) over the interior
 // cells (one thread per cell), with the fused next-step CFL minimum into
 // dtmin when fuse.
 void warp_stage(int nd, bool mixed, int mode, bool hang, bool fuse, const double* qin, double* out,
