@@ -102,7 +102,8 @@ struct h3c_solver_s {
   long long stage_cap = 0;
   double* d_adj = nullptr;  // adjoint workspace (checkpoints, stage states, cotangents), kept between calls
   size_t adj_cap = 0;
-  long long* d_dev2caller = nullptr;
+  int* d_dev2caller = nullptr;  // nullptr: the caller's numbering is the internal one
+  int* d_dev2caller_mem = nullptr;
   std::vector<long long> dev2caller, caller2dev;
   Scalars* d_sc = nullptr;
   Scalars* h_sc = nullptr;  // pinned host copy of instance 0's scalars (the per-step dt read-back)
@@ -217,7 +218,8 @@ void free_grid(h3c_solver s) {
   dfree(s->d_nbr); dfree(s->d_lvl); dfree(s->d_sub); dfree(s->d_gbndry); dfree(s->d_gpos);
   dfree(s->d_gapply); dfree(s->d_gown); dfree(s->d_gdx); dfree(s->d_gpartner); dfree(s->d_xc);
   dfree(s->d_bcs); dfree(s->d_q[0]); dfree(s->d_q[1]); dfree(s->d_q[2]); dfree(s->d_slopes); dfree(s->d_stage);
-  dfree(s->d_dev2caller);
+  dfree(s->d_dev2caller_mem);
+  s->d_dev2caller = nullptr;
   dfree(s->d_vel);
   s->vel_set = false;
   dfree(s->d_blk_inst); dfree(s->d_inst_end); dfree(s->d_ginst);
@@ -350,27 +352,34 @@ void launch_bc_ptr(h3c_solver s, double* q, const double* qlhs, const StepBegin&
 void launch_bc(h3c_solver s, int which) { launch_bc_ptr(s, s->d_q[which], s->d_q[0]); }
 
 template <int ND, int PHYS>
-void launch_cfl_t(h3c_solver s, long long* slot) {
+void launch_cfl_t(h3c_solver s, long long* slot, const double* src, long long src_ld) {
   Launch L(s, K_CFL);
-  k_cfl<ND, PHYS><<<blocks(s->n_int), kBlock, 0, s->stream>>>(s->d_q[0], geometry(s), s->pc, slot, s->d_sc);
+  if (src)
+    launch_chain(k_cfl<ND, PHYS, true>, blocks(s->n_tot), kBlock, 0, s->stream, s->d_q[0], geometry(s), s->pc, slot,
+                 s->d_sc, src, src_ld, s->d_dev2caller);
+  else
+    launch_chain(k_cfl<ND, PHYS, false>, blocks(s->n_int), kBlock, 0, s->stream, s->d_q[0], geometry(s), s->pc, slot,
+                 s->d_sc, nullptr, 0, nullptr);
 }
-void launch_cfl(h3c_solver s, long long* slot) {
+// The minimum cell time step of lhs into slot; src: columns (device memory,
+// caller numbering) that lhs is read from first.  clear: slot still holds an older minimum.
+void launch_cfl(h3c_solver s, long long* slot, const double* src = nullptr, long long src_ld = 0, bool clear = true) {
   if (s->desc.physics == H3C_ADVECTION && !s->vel_set) return;  // no velocity yet: no time step
   s->mirror_valid = false;  // the pass checks every cell
-  {
+  if (clear) {
     Launch L(s, K_SCALAR);
-    k_reset_slot<<<blocks(s->n_inst), kBlock, 0, s->stream>>>(slot, s->n_inst);
+    launch_chain(k_reset_slot, blocks(s->n_inst), kBlock, 0, s->stream, slot, s->n_inst);
   }
   if (s->nd == 2) {
-    if (s->desc.physics == H3C_EULER) launch_cfl_t<2, EULER>(s, slot);
-    else if (s->desc.physics == H3C_CNS) launch_cfl_t<2, CNS>(s, slot);
-    else if (s->desc.physics == H3C_ADVECTION) launch_cfl_t<2, ADVECTION>(s, slot);
-    else launch_cfl_t<2, HEAT>(s, slot);
+    if (s->desc.physics == H3C_EULER) launch_cfl_t<2, EULER>(s, slot, src, src_ld);
+    else if (s->desc.physics == H3C_CNS) launch_cfl_t<2, CNS>(s, slot, src, src_ld);
+    else if (s->desc.physics == H3C_ADVECTION) launch_cfl_t<2, ADVECTION>(s, slot, src, src_ld);
+    else launch_cfl_t<2, HEAT>(s, slot, src, src_ld);
   } else {
-    if (s->desc.physics == H3C_EULER) launch_cfl_t<3, EULER>(s, slot);
-    else if (s->desc.physics == H3C_CNS) launch_cfl_t<3, CNS>(s, slot);
-    else if (s->desc.physics == H3C_ADVECTION) launch_cfl_t<3, ADVECTION>(s, slot);
-    else launch_cfl_t<3, HEAT>(s, slot);
+    if (s->desc.physics == H3C_EULER) launch_cfl_t<3, EULER>(s, slot, src, src_ld);
+    else if (s->desc.physics == H3C_CNS) launch_cfl_t<3, CNS>(s, slot, src, src_ld);
+    else if (s->desc.physics == H3C_ADVECTION) launch_cfl_t<3, ADVECTION>(s, slot, src, src_ld);
+    else launch_cfl_t<3, HEAT>(s, slot, src, src_ld);
   }
 }
 
@@ -804,7 +813,7 @@ static int prepare_instance(h3c_solver s, int k, const h3c_grid* gr, InstanceTab
 __global__ void k_check_tables(const int* __restrict__ nbr, const int* __restrict__ sub,
                                const int* __restrict__ gbndry, const unsigned char* __restrict__ lvl,
                                const int* __restrict__ hids, int hid_mask, long long nhids,
-                               const long long* __restrict__ dev2caller, long long n_int, long long n_tot,
+                               const int* __restrict__ dev2caller, long long n_int, long long n_tot,
                                long long ld, long long nsub, int np, int nsubc, long long ng, int nlev,
                                unsigned long long* bad) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1021,7 +1030,7 @@ static int set_grids(h3c_solver s, int ninst, const h3c_grid* grids) {
   if (s->desc.time_integration == H3C_SSPRK3) H3C_CUDA(s, cudaMalloc(&s->d_q[2], sizeof(double) * s->nv * L));
   if (s->desc.physics == H3C_CNS || s->desc.reconstruction == H3C_RECON_MUSCL)
     H3C_CUDA(s, cudaMalloc(&s->d_slopes, sizeof(double) * nd * s->nv * L));
-  H3C_CUDA(s, cudaMalloc(&s->d_dev2caller, sizeof(long long) * n_tot));
+  H3C_CUDA(s, cudaMalloc(&s->d_dev2caller_mem, sizeof(int) * n_tot));
   if (ninst > 1) {
     H3C_CUDA(s, cudaMalloc(&s->d_blk_inst, sizeof(int) * h_blk.size()));
     H3C_CUDA(s, cudaMalloc(&s->d_inst_end, sizeof(long long) * ninst));
@@ -1110,7 +1119,16 @@ static int set_grids(h3c_solver s, int ninst, const h3c_grid* grids) {
     }
   }
   H3C_CUDA(s, cudaMemcpy(s->d_bcs, s->h_bcs.data(), sizeof(BcParam) * s->h_bcs.size(), cudaMemcpyHostToDevice));
-  H3C_CUDA(s, cudaMemcpy(s->d_dev2caller, dev2caller.data(), sizeof(long long) * n_tot, cudaMemcpyHostToDevice));
+  {
+    std::vector<int> map(n_tot);
+    bool same = n_tot == ncaller;
+    for (long long i = 0; i < n_tot; ++i) {
+      map[i] = (int)dev2caller[i];
+      same = same && dev2caller[i] == i;
+    }
+    H3C_CUDA(s, cudaMemcpy(s->d_dev2caller_mem, map.data(), sizeof(int) * n_tot, cudaMemcpyHostToDevice));
+    s->d_dev2caller = same ? nullptr : s->d_dev2caller_mem;
+  }
   H3C_CUDA(s, cudaMemset(s->d_q[0], 0, sizeof(double) * s->nv * L));
   H3C_CUDA(s, cudaMemset(s->d_q[1], 0, sizeof(double) * s->nv * L));
   if (s->d_q[2]) H3C_CUDA(s, cudaMemset(s->d_q[2], 0, sizeof(double) * s->nv * L));
@@ -1129,7 +1147,7 @@ static int set_grids(h3c_solver s, int ninst, const h3c_grid* grids) {
     const long long span = std::max({n_int, nsub, ng, nh, 1LL});
     const int hid_mask = halo_tables ? kHaloCellMask : -1;  // Euler entries carry a direction and a side
     k_check_tables<<<blocks(span), kBlock, 0, s->stream>>>(s->d_nbr, s->d_sub, s->d_gbndry, s->d_lvl, s->d_hids,
-                                                           hid_mask, nh, s->d_dev2caller, n_int, n_tot, L, nsub,
+                                                           hid_mask, nh, s->d_dev2caller_mem, n_int, n_tot, L, nsub,
                                                            np, nsubc, ng,
                                                            s->nlev, d_bad);
     unsigned long long bad = 0;
@@ -1163,6 +1181,41 @@ static int ready(h3c_solver s, const char* what) {
   return H3C_OK;
 }
 
+// Whether the span of the caller's columns q [nv][ld] lies in this device's
+// memory, whole inside one allocation, and apart from the solver's own
+// buffers: the kernels then read or write it in place.  Anything else goes
+// through the staging buffer and cudaMemcpy, which checks for itself.
+static bool in_place(h3c_solver s, const double* q, int64_t ld) {
+  if ((uintptr_t)q & 7) return false;
+  cudaPointerAttributes at{};
+  int dev = 0;
+  if (cudaPointerGetAttributes(&at, q) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (at.type != cudaMemoryTypeDevice || at.device != dev) return false;
+  using Range_t = int (*)(unsigned long long*, size_t*, unsigned long long);
+  static const Range_t range = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult r;
+    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &r) != cudaSuccess ||
+        r != cudaDriverEntryPointSuccess)
+      fn = nullptr;
+    cudaGetLastError();
+    return (Range_t)fn;
+  }();
+  unsigned long long base = 0;
+  size_t size = 0;
+  const unsigned long long lo = (unsigned long long)(uintptr_t)q;
+  const unsigned long long hi = lo + 8ULL * ((s->nv - 1) * (unsigned long long)ld + s->n_caller);
+  if (!range || range(&base, &size, lo) != 0 || hi > base + size) return false;
+  for (const double* own : s->d_q) {
+    const unsigned long long o = (unsigned long long)(uintptr_t)own;
+    if (own && lo < o + 8ULL * s->nv * s->ld && o < hi) return false;
+  }
+  return true;
+}
+
 static int ensure_stage(h3c_solver s, long long ld) {
   const long long need = (long long)s->nv * ld;
   if (need > s->stage_cap) {
@@ -1178,14 +1231,18 @@ int h3c_set_state(h3c_solver s, int which, const double* q, int64_t ld) {
   if (!s->has_grid) return s->fail(H3C_E_STATE, "h3c_set_state: no grid");
   const long long nc = s->n_caller;
   if (ld < nc) return s->fail(H3C_E_INVALID, "h3c_set_state: ld < n_cells");
-  int rc = ensure_stage(s, nc);
-  if (rc) return rc;
-  for (int v = 0; v < s->nv; ++v)  // q in host or device memory (unified addressing)
-    H3C_CUDA(s, cudaMemcpyAsync(s->d_stage + v * nc, q + v * ld, sizeof(double) * nc, cudaMemcpyDefault,
-                                s->stream));
-  k_gather<<<blocks(s->n_tot), kBlock, 0, s->stream>>>(s->d_stage, nc, s->d_q[which], s->ld, s->d_dev2caller,
-                                                       s->n_tot, s->nv);
-  if (which == 0) launch_cfl(s, &s->d_sc->dtmin_ord);
+  if (!in_place(s, q, ld)) {
+    if (int rc = ensure_stage(s, nc)) return rc;
+    for (int v = 0; v < s->nv; ++v)  // q in host or device memory (unified addressing)
+      H3C_CUDA(s, cudaMemcpyAsync(s->d_stage + v * nc, q + v * ld, sizeof(double) * nc, cudaMemcpyDefault,
+                                  s->stream));
+    q = s->d_stage;
+    ld = nc;
+  }
+  if (which == 0 && !(s->desc.physics == H3C_ADVECTION && !s->vel_set))
+    launch_cfl(s, &s->d_sc->dtmin_ord, q, ld);
+  else
+    k_gather<<<blocks(s->n_tot), kBlock, 0, s->stream>>>(q, ld, s->d_q[which], s->ld, s->d_dev2caller, s->n_tot, s->nv);
   H3C_CUDA(s, cudaStreamSynchronize(s->stream));
   return s->cuda(cudaGetLastError(), "h3c_set_state");
 }
@@ -1234,7 +1291,7 @@ int h3c_write_vtk(h3c_solver s, const char* fname, const h3c_grid* grid, const i
   auto download = [&](const double* src, int cols, std::vector<double>& out) -> int {
     double* tmp = nullptr;
     H3C_CUDA(s, cudaMalloc(&tmp, sizeof(double) * cols * n));
-    k_scatter<<<blocks(s->n_tot), kBlock, 0, s->stream>>>(src, s->ld, tmp, n, s->d_dev2caller, s->n_tot, cols);
+    k_scatter<<<blocks(s->n_tot), kBlock, 0, s->stream>>>(src, s->ld, tmp, n, s->d_dev2caller, s->n_tot, s->n_tot, cols);
     out.resize((size_t)cols * n);
     cudaMemcpyAsync(out.data(), tmp, sizeof(double) * cols * n, cudaMemcpyDeviceToHost, s->stream);
     const cudaError_t e = cudaStreamSynchronize(s->stream);
@@ -1361,11 +1418,13 @@ int h3c_get_state(h3c_solver s, int which, double* q, int64_t ld) {
   if (!s->has_grid) return s->fail(H3C_E_STATE, "h3c_get_state: no grid");
   const long long nc = s->n_caller;
   if (ld < nc) return s->fail(H3C_E_INVALID, "h3c_get_state: ld < n_cells");
-  int rc = ensure_stage(s, nc);
-  if (rc) return rc;
-  k_scatter<<<blocks(s->n_tot), kBlock, 0, s->stream>>>(s->d_q[which], s->ld, s->d_stage, nc, s->d_dev2caller,
-                                                        s->n_tot, s->nv);
-  for (int v = 0; v < s->nv; ++v)  // q in host or device memory (unified addressing)
+  const bool direct = in_place(s, q, ld);
+  if (!direct) {
+    if (int rc = ensure_stage(s, nc)) return rc;
+  }
+  k_scatter<<<blocks(s->n_tot), kBlock, 0, s->stream>>>(s->d_q[which], s->ld, direct ? q : s->d_stage, direct ? ld : nc,
+                                                        s->d_dev2caller, s->n_tot, s->n_tot, s->nv);
+  for (int v = 0; v < s->nv && !direct; ++v)  // q in host or device memory (unified addressing)
     H3C_CUDA(s, cudaMemcpyAsync(q + v * ld, s->d_stage + v * nc, sizeof(double) * nc, cudaMemcpyDefault,
                                 s->stream));
   H3C_CUDA(s, cudaStreamSynchronize(s->stream));
@@ -1408,8 +1467,8 @@ int h3c_reset_time(h3c_solver s) {
   s->stage_next = 0;  // a step run by parts starts over
   s->mirror_valid = false;
   k_init_time<<<blocks(s->n_inst), kBlock, 0, s->stream>>>(s->d_sc, s->desc.time_end, s->n_inst, s->h_mirror);
-  launch_cfl(s, &s->d_sc->dtmin_ord);
-  k_set_dt<<<blocks(s->n_inst), kBlock, 0, s->stream>>>(s->d_sc, 0, s->n_inst);
+  launch_cfl(s, &s->d_sc->dtmin_ord, nullptr, 0, false);  // k_init_time cleared the slot
+  launch_chain(k_set_dt, blocks(s->n_inst), kBlock, 0, s->stream, s->d_sc, 0, s->n_inst);
   return s->cuda(cudaGetLastError(), "h3c_reset_time");
 }
 
@@ -2250,6 +2309,32 @@ int h3c_solve_dt(h3c_solver s, int64_t nsteps, const double* dts) {
   return s->cuda(cudaGetLastError(), "h3c_solve_dt");
 }
 
+// An adjoint's cotangent columns (caller numbering, host or device memory)
+// into the interior cells of dst, and a gradient back (ghosts zero).
+static int caller_to_internal(h3c_solver s, const double* src, double* dst) {
+  const long long nc = s->n_caller;
+  if (!in_place(s, src, nc)) {
+    if (int rc = ensure_stage(s, nc)) return rc;
+    cudaMemcpyAsync(s->d_stage, src, sizeof(double) * s->nv * nc, cudaMemcpyDefault, s->stream);
+    src = s->d_stage;
+  }
+  k_gather<<<blocks(s->n_int), kBlock, 0, s->stream>>>(src, nc, dst, s->ld, s->d_dev2caller, s->n_int, s->nv);
+  ++s->launches;
+  return H3C_OK;
+}
+static int internal_to_caller(h3c_solver s, const double* src, double* dst) {
+  const long long nc = s->n_caller;
+  const bool direct = in_place(s, dst, nc);
+  if (!direct) {
+    if (int rc = ensure_stage(s, nc)) return rc;
+  }
+  k_scatter<<<blocks(s->n_tot), kBlock, 0, s->stream>>>(src, s->ld, direct ? dst : s->d_stage, nc, s->d_dev2caller,
+                                                        s->n_tot, s->n_int, s->nv);
+  ++s->launches;
+  if (!direct) cudaMemcpyAsync(dst, s->d_stage, sizeof(double) * s->nv * nc, cudaMemcpyDefault, s->stream);
+  return H3C_OK;
+}
+
 // Backward sweep of the discrete adjoint.  Memory: nck checkpoints + the
 // stage states of one segment + 3 work + 3 cotangent states.  The forward
 // stores the stage states of the last segment as it goes, so that segment
@@ -2273,7 +2358,9 @@ int h3c_adjoint(h3c_solver s, int64_t nsteps, int64_t every, const double* dJ_dq
     return sizeof(double) * ((size_t)Q * (nck + per * ev + 7) + nsteps + extra_m);
   };
   if (every > nsteps) every = nsteps;
-  if (every == 0) {  // no recomputation if that fits in half of the free memory, else ~sqrt(N) segments
+  if (every == 0 && need(nsteps) <= s->adj_cap) {
+    every = nsteps;  // the workspace of an earlier call holds it: no query of the free memory
+  } else if (every == 0) {  // no recomputation if that fits in half of the free memory, else ~sqrt(N) segments
     size_t fr = 0, tot = 0;
     cudaMemGetInfo(&fr, &tot);
     const size_t budget = fr / 2 + s->adj_cap;
@@ -2322,13 +2409,7 @@ int h3c_adjoint(h3c_solver s, int64_t nsteps, int64_t every, const double* dJ_dq
   double* lamC = lam + 2 * Q;  // last-stage input cotangent (RK2, SSP-RK3)
   double* lamD = lam + 3 * Q;  // first-stage output cotangent (SSP-RK3)
   cudaMemsetAsync(lam, 0, sizeof(double) * Q * 4, s->stream);
-  if (int rc = ensure_stage(s, s->n_caller)) return rc;
-  // host or device arrays (unified addressing)
-  for (int v = 0; v < nv; ++v)
-    cudaMemcpyAsync(s->d_stage + v * s->n_caller, dJ_dqN + v * s->n_caller, sizeof(double) * s->n_caller,
-                    cudaMemcpyDefault, s->stream);
-  k_gather<<<blocks(s->n_int), kBlock, 0, s->stream>>>(s->d_stage, s->n_caller, lamA, L, s->d_dev2caller, s->n_int, (int)nv);
-  ++s->launches;
+  if (int rc = caller_to_internal(s, dJ_dqN, lamA)) return rc;
   auto adj = [&](const double* qin, const double* lamin, double* gout, double alpha, double beta,
                  const double* extra = nullptr, double gam = 0.0, const double* extra2 = nullptr,
                  double gam2 = 0.0) {
@@ -2442,12 +2523,7 @@ int h3c_adjoint(h3c_solver s, int64_t nsteps, int64_t every, const double* dJ_dq
     }
   }
   // ---- gradient (internal -> caller numbering), dt sequence ----
-  cudaMemsetAsync(s->d_stage, 0, sizeof(double) * nv * s->n_caller, s->stream);
-  k_scatter<<<blocks(s->n_int), kBlock, 0, s->stream>>>(lamA, L, s->d_stage, s->n_caller, s->d_dev2caller, s->n_int, (int)nv);
-  ++s->launches;
-  for (int v = 0; v < nv; ++v)
-    cudaMemcpyAsync(dJ_dq0 + v * s->n_caller, s->d_stage + v * s->n_caller, sizeof(double) * s->n_caller,
-                    cudaMemcpyDefault, s->stream);
+  if (int rc = internal_to_caller(s, lamA, dJ_dq0)) return rc;
   if (dts_out) cudaMemcpyAsync(dts_out, d_dts, sizeof(double) * nsteps, cudaMemcpyDefault, s->stream);
   // the solver is left at step N with the scalars of the forward run
   cudaStreamSynchronize(s->stream);
@@ -2489,24 +2565,6 @@ __global__ void k_cht_fluid_to_heat(const double* __restrict__ tbar, GhostTables
   const int Q = gtf.partner[i];
   if (Q < 0) return;
   atomicAdd(lams + Q, tbar[i]);
-}
-
-static void caller_to_internal(h3c_solver s, const double* src, double* dst) {
-  for (int v = 0; v < s->nv; ++v)
-    cudaMemcpyAsync(s->d_stage + v * s->n_caller, src + v * s->n_caller, sizeof(double) * s->n_caller,
-                    cudaMemcpyDefault, s->stream);
-  k_gather<<<blocks(s->n_int), kBlock, 0, s->stream>>>(s->d_stage, s->n_caller, dst, s->ld, s->d_dev2caller, s->n_int,
-                                                       s->nv);
-  ++s->launches;
-}
-static void internal_to_caller(h3c_solver s, const double* src, double* dst) {
-  cudaMemsetAsync(s->d_stage, 0, sizeof(double) * s->nv * s->n_caller, s->stream);
-  k_scatter<<<blocks(s->n_int), kBlock, 0, s->stream>>>(src, s->ld, s->d_stage, s->n_caller, s->d_dev2caller, s->n_int,
-                                                        s->nv);
-  ++s->launches;
-  for (int v = 0; v < s->nv; ++v)
-    cudaMemcpyAsync(dst + v * s->n_caller, s->d_stage + v * s->n_caller, sizeof(double) * s->n_caller,
-                    cudaMemcpyDefault, s->stream);
 }
 
 int h3c_cht_adjoint(h3c_solver cns, h3c_solver heat, double Tr0, int64_t nsteps, int64_t every,
@@ -2611,8 +2669,8 @@ int h3c_cht_adjoint(h3c_solver cns, h3c_solver heat, double Tr0, int64_t nsteps,
   double *lfA = lf, *lfB = lf + Qf, *lfT = lf + 2 * Qf, *lsA = ls, *lsB = ls + Qs;
   cudaMemsetAsync(lf, 0, sizeof(double) * 3 * Qf, st);
   cudaMemsetAsync(ls, 0, sizeof(double) * 2 * Qs, st);
-  caller_to_internal(cns, dJ_dqN, lfA);
-  caller_to_internal(heat, dJ_dTN, lsA);
+  for (const int rc : {caller_to_internal(cns, dJ_dqN, lfA), caller_to_internal(heat, dJ_dTN, lsA)})
+    if (rc) { cudaFree(ws); return rc; }
   const Geometry gf = geometry(cns), gs = geometry(heat);
   const GhostTables gtf = ghosts(cns), gts = ghosts(heat);
   const unsigned nbf = (unsigned)blocks(cns->n_int), nbs = (unsigned)blocks(heat->n_int);
@@ -2710,8 +2768,12 @@ int h3c_cht_adjoint(h3c_solver cns, h3c_solver heat, double Tr0, int64_t nsteps,
       bwd_seg(i1 - i0);
     }
   }
-  internal_to_caller(cns, lfA, dJ_dq0);
-  internal_to_caller(heat, lsA, dJ_dT0);
+  for (const int rc : {internal_to_caller(cns, lfA, dJ_dq0), internal_to_caller(heat, lsA, dJ_dT0)})
+    if (rc) {
+      cudaStreamSynchronize(st);
+      cudaFree(ws);
+      return rc;
+    }
   if (dts) {
     cudaMemcpyAsync(dts, dtf, sizeof(double) * nsteps, cudaMemcpyDefault, st);
     cudaMemcpyAsync(dts + nsteps, dth, sizeof(double) * nsteps, cudaMemcpyDefault, st);
