@@ -1102,6 +1102,130 @@ __global__ void __launch_bounds__(kBlock) k_stage(const double* __restrict__ qin
 }
 
 // ---------------------------------------------------------------------------
+// Stage of the scalar physics (heat, advection) on one grid without
+// coarse/fine faces: the fluxes, update and fused CFL minimum of k_stage, two
+// neighbouring cells of the Morton order per thread.  A cell reads little and
+// computes less, so the stage is bound by how many loads are in flight: the
+// pair's rows come as vector loads (8 bytes of neighbour indices, 16 of state
+// and velocity), the neighbours of both cells are all requested before any
+// flux, a neighbour that is the pair's other cell is not loaded at all, and
+// dt / length is divided once per level and block.  2048^2 advection, LLF,
+// forward Euler: 73.8 us per stage in k_stage -> 59.4 here; 100^3 heat: 16.9
+// -> 14.8 (with the events' overhead of about 5).  What is left is latency:
+// 3.4 TB/s of DRAM traffic, issue slots and L1 under half used.  Prefetching
+// the tables of a block one wave ahead into L2 gained 3% in advection and
+// lost 8% in heat; left out.
+// ---------------------------------------------------------------------------
+template <int ND, int PHYS, int FLUX, int MODE, bool FUSE>
+__global__ void __launch_bounds__(kBlock) k_stage_scalar(const double* __restrict__ qin, double* out, Geometry g,
+                                                         PhysConst pc, const Scalars* __restrict__ sc,
+                                                         long long* dtmin) {
+  static_assert(PHYS == HEAT || PHYS == ADVECTION, "one variable");
+  constexpr bool ADV = PHYS == ADVECTION;
+  __shared__ double skdt[kMaxLevels], sidx[kMaxLevels];  // dt / length, 1 / length
+  chain_begin();
+  if (threadIdx.x < kMaxLevels) {
+    skdt[threadIdx.x] = sc->dt / g.len[threadIdx.x];
+    if (!ADV) sidx[threadIdx.x] = 1 / g.len[threadIdx.x];
+  }
+  const long long ld = g.ld;
+  const long long c = 2 * ((long long)blockIdx.x * kBlock + threadIdx.x);
+  const bool live = c < g.n_int, both = c + 1 < g.n_int;  // rows are padded to 32 cells: the pair's loads stay inside
+  int2 nb[2 * ND];
+  double2 q = make_double2(0.0, 0.0), u[ND], q0 = q;
+  uchar2 lv = make_uchar2(0, 0);
+  if (live) {
+#pragma unroll
+    for (int p = 0; p < 2 * ND; ++p) nb[p] = __ldg(reinterpret_cast<const int2*>(g.nbr + p * ld + c));
+    q = __ldg(reinterpret_cast<const double2*>(qin + c));
+    lv = __ldg(reinterpret_cast<const uchar2*>(g.lvl + c));
+    if (ADV) {
+#pragma unroll
+      for (int d = 0; d < ND; ++d) u[d] = __ldg(reinterpret_cast<const double2*>(g.vel + d * ld + c));
+    }
+    if (MODE != 0) q0 = *reinterpret_cast<const double2*>(g.q0 + c);
+    if (!both) {  // the last cell of an odd count: its partner repeats it
+#pragma unroll
+      for (int p = 0; p < 2 * ND; ++p) nb[p].y = nb[p].x;
+    }
+  }
+  double qn[2 * ND][2], un[ADV ? 2 * ND : 1][2];
+  if (live) {
+#pragma unroll
+    for (int p = 0; p < 2 * ND; ++p) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int n = j ? nb[p].y : nb[p].x;
+        const bool pair = both && (j ? n == (int)c : n == (int)c + 1);
+        qn[p][j] = pair ? (j ? q.x : q.y) : __ldg(qin + n);
+        if (ADV) un[p][j] = pair ? (j ? u[p >> 1].x : u[p >> 1].y) : __ldg(g.vel + (p >> 1) * ld + n);
+      }
+    }
+  }
+  __syncthreads();  // the level tables; every load has been issued
+  long long ord = kOrdMax;
+  bool bad = false;
+  if (live) {
+    double o[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const double qc = j ? q.y : q.x;
+      const int l = j ? lv.y : lv.x;
+      double acc = 0.0;
+#pragma unroll
+      for (int d = 0; d < ND; ++d) {
+        double fm, fp;
+        if (ADV) {
+          // advection/physics.hpp:120-145 (k_stage)
+          auto flux = [&](double qL, double qR, double uL, double uR) {
+            if (FLUX == LLF) {
+              const double lambda_max = fmax(fabs(uL), fabs(uR));
+              return 0.5 * (qL * uL + qR * uR + lambda_max * (qL - qR));
+            }
+            const double u_srfc = 0.5 * (uL + uR);
+            const double f = uL * qL;
+            return u_srfc < 0 ? f * -1. : f;
+          };
+          const double uc = j ? u[d].y : u[d].x;
+          fm = flux(qn[2 * d][j], qc, un[2 * d][j], uc);
+          fp = flux(qc, qn[2 * d + 1][j], uc, un[2 * d + 1][j]);
+        } else {
+          // three_point: heat/physics.hpp:113-119
+          fm = sidx[l] * (qn[2 * d][j] - qc);
+          fp = sidx[l] * (qc - qn[2 * d + 1][j]);
+        }
+        acc = acc + (fm - fp);
+      }
+      o[j] = rk_combine<MODE>(MODE == 0 ? 0.0 : (j ? q0.y : q0.x), qc, skdt[l] * acc);
+    }
+    if (both) *reinterpret_cast<double2*>(out + c) = make_double2(o[0], o[1]);
+    else out[c] = o[0];
+    if (FUSE) {
+      // cell_dt of both cells; on one level the faster cell's is the smaller (a division is monotonic)
+      bad = !isfinite(o[0]) || (both && !isfinite(o[1]));
+      double ua[ND], ub[ND];
+      if (ADV) {
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+          ua[d] = lv.x == lv.y && both ? fmax(fabs(u[d].x), fabs(u[d].y)) : u[d].x;
+          ub[d] = u[d].y;
+        }
+      }
+      const double ca = cell_dt<ND, PHYS>(o, g.len[lv.x], pc, ua);
+      if (!isnan(ca)) ord = dbl_to_ord(ca);
+      if (both && lv.x != lv.y) {
+        const double cb = cell_dt<ND, PHYS>(o + 1, g.len[lv.y], pc, ub);
+        if (!isnan(cb)) ord = min(ord, dbl_to_ord(cb));
+      }
+    }
+  }
+  if (FUSE) {
+    flag_bad_state(bad, sc, 0);
+    block_min_atomic(ord, dtmin);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Tile stage kernel (Euler).  A block owns kBlock consecutive cells of the
 // Morton order, which form a compact brick of the grid.  Primitive variables
 // are computed once per cell into shared memory, each cell evaluates the flux

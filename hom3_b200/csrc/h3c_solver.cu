@@ -494,6 +494,16 @@ void stage_t(h3c_solver s, const double* qin, double* out) {
         qin, out, geometry(s), s->pc, s->d_sc, &s->d_sc->dtmin_ord);
     return;
   }
+  // one grid without coarse/fine faces: two cells per thread (neighbour entries are cells then, never groups)
+  if constexpr ((PHYS == HEAT || PHYS == ADVECTION) && !HANG) {
+    // from one full wave of k_stage's blocks on; below, a thread per cell finishes sooner (32,768 heat cells:
+    // 7.0 us against 8.5)
+    if (s->n_inst == 1 && s->n_int >= 6LL * kBlock * num_sms()) {
+      launch_chain(k_stage_scalar<ND, PHYS, FLUX, MODE, FUSE>, blocks((s->n_int + 1) / 2), kBlock, 0, s->stream, qin, out,
+                   geometry(s), s->pc, s->d_sc, &s->d_sc->dtmin_ord);
+      return;
+    }
+  }
   launch_chain(k_stage<ND, PHYS, FLUX, R, MODE, HANG, FUSE>, blocks(s->n_int), kBlock, 0, s->stream, qin, out,
                s->d_slopes, geometry(s), s->pc, s->d_sc, &s->d_sc->dtmin_ord);
 }
