@@ -304,6 +304,10 @@ template <class R> __device__ __forceinline__ R p_int(R s, R M) {
   return fabs(M) > R(1) ? sup : (R(0.25) * ((M + s) * (M + s))) * (R(2) - s * M);
 }
 
+// |M| >= 1 or NaN, from the exponent bits (at exactly 1 the subsonic and supersonic splits agree)
+__device__ __forceinline__ bool beyond_one(double M) { return (__double2hiint(M) & 0x7fffffff) >= 0x3ff00000; }
+__device__ __forceinline__ bool beyond_one(float M) { return (__float_as_int(M) & 0x7fffffff) >= 0x3f800000; }
+
 // AUSM (Liou-Steffen): euler/physics.hpp:276-293, theta_ :315-325
 template <class R, int ND>
 __device__ __forceinline__ void ausm(const Prim<R, ND>& L, const Prim<R, ND>& Rt, int d, R* f) {

@@ -138,6 +138,7 @@ struct h3c_solver_s {
   // CNS tile kernel (h3c_stage_cns.cu): its tables reuse d_lnb / d_hids / d_hoff
   bool cns_ok = false;
   int* d_h1end = nullptr;
+  unsigned *d_blist = nullptr, *d_bsel = nullptr;  // brick grids: border lists
   unsigned short* d_hnb = nullptr;
   double* d_gsl = nullptr;  // ghost slopes [nd * nv][ngl]
   long long ngl = 0;
@@ -224,7 +225,7 @@ void free_grid(h3c_solver s) {
   s->vel_set = false;
   dfree(s->d_blk_inst); dfree(s->d_inst_end); dfree(s->d_ginst);
   dfree(s->d_lnb); dfree(s->d_hids); dfree(s->d_hoff); dfree(s->d_goff); dfree(s->d_grp);
-  dfree(s->d_h1end); dfree(s->d_hnb); dfree(s->d_gsl);
+  dfree(s->d_h1end); dfree(s->d_hnb); dfree(s->d_gsl); dfree(s->d_blist); dfree(s->d_bsel);
   dfree(s->d_pack);
   dfree(s->d_gsrc);
   s->mirror_valid = false;
@@ -417,7 +418,7 @@ void stage_t(h3c_solver s, const double* qin, double* out) {
     int grid = s->persist_blocks > 0 ? s->persist_blocks : s->cns_bps * num_sms();
     grid = (int)std::max<long long>(1, std::min<long long>(grid, s->ntiles));
     const CnsHaloGeom ch{HaloGeom{s->d_lnb, s->d_hids, s->d_hoff, s->d_grp, s->d_goff, s->hmax}, s->d_h1end, s->d_hnb,
-                         s->d_gsl, s->ngl, s->h1max};
+                         s->d_gsl, s->ngl, s->h1max, s->d_blist, s->d_bsel};
     if (s->ng > 0) s->launches++;  // the ghost-slope pass
     cns_halo_stage(ND, std::is_same<R, float>::value, MODE, FUSE, qin, out, geometry(s), ghosts(s), ch, s->pc,
                    s->d_sc, &s->d_sc->dtmin_ord, &s->d_sc->status, grid, s->cns_smem, s->stream, s->d_gsl);
@@ -1102,8 +1103,20 @@ static int set_grids(h3c_solver s, int ninst, const h3c_grid* grids) {
     s->warp_bps = warp_prepare(nd, s->desc.precision == H3C_MIXED);
   if (cns_tables) {
     const bool mixed = s->desc.precision == H3C_MIXED;
-    const size_t smem = cns_halo_smem_bytes(nd, mixed, CH.base.hmax, CH.h1max);
-    const int bps = smem <= 227 * 1024 ? cns_halo_prepare(nd, mixed, smem) : 0;
+    // the brick variant where every tile is one; a grid of a few tiles may fit only the general one
+    size_t smem = 0;
+    int bps = 0;
+    for (int brick = CH.brick ? 1 : 0; brick >= 0 && bps == 0; --brick) {
+      CH.brick = brick != 0;
+      smem = cns_halo_smem_bytes(nd, mixed, CH.base.hmax, CH.h1max, CH.brick);
+      bps = smem <= 227 * 1024 ? cns_halo_prepare(nd, mixed, smem, CH.brick) : 0;
+    }
+    if (bps > 0 && CH.brick) {
+      H3C_CUDA(s, cudaMalloc(&s->d_blist, sizeof(unsigned) * CH.blist.size()));
+      H3C_CUDA(s, cudaMalloc(&s->d_bsel, sizeof(unsigned) * CH.bsel.size()));
+      H3C_CUDA(s, cudaMemcpy(s->d_blist, CH.blist.data(), sizeof(unsigned) * CH.blist.size(), cudaMemcpyHostToDevice));
+      H3C_CUDA(s, cudaMemcpy(s->d_bsel, CH.bsel.data(), sizeof(unsigned) * CH.bsel.size(), cudaMemcpyHostToDevice));
+    }
     if (bps > 0) {
       const HaloHost& B = CH.base;
       s->ngl = std::max<long long>(1, (ng + 31) / 32 * 32);

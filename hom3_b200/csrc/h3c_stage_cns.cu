@@ -72,29 +72,98 @@ __global__ void __launch_bounds__(kBlock) k_ghost_slopes(const double* __restric
 // (cns/physics.hpp:305-338 reads no energy slope), [sd][v] for v <= nd.
 template <int ND> constexpr int kCnsSlopeVars = ND + 1;
 
+// Whether the tables are a "brick" grid's: every tile a whole Morton brick, or
+// at least with no more layer-1 cells than one (H1 of them: 256 around 8x8x4
+// cells, 64 around 16x16) and no more faces whose minus side lies outside the
+// tile than fit its border list (kCnsBorder: 32 + 32 + 64 of an 8x8x4 brick,
+// 16 + 16 of a 16x16 one, each direction's padded to whole warps).  Bricks
+// take the kernel variant with constant row strides and the border list.
+template <int ND> constexpr int kCnsBrickH1 = ND == 3 ? 256 : 64;
+template <int ND> constexpr int kCnsBorder = ND == 3 ? 128 : 64;
+
 // Shared memory of one block.  In FP64 the copies land in the primitive
 // rows themselves (the tile and first-layer cells' states are the first nv
 // rows of the primitives) and only the second layer has a landing area of
 // its own; in FP32 (R = float) the FP64 states land in a separate area.
-//   mbarrier (16) | [FP32: landing [nv][S] f64] | primitives [nv + nd + 2][S1] R |
-//   [FP64: second-layer landing [nv][S - S1] f64] | slopes [nd (nd + 1)][S1] R |
-//   plus fluxes [nv][256] f64 | neighbour slots [2][2nd][256] u16
+//   mbarrier (16) | plus fluxes [nv][256] f64 | primitives [nv + nd + 2][S1] R | slopes [nd (nd + 1)][S1] R |
+//   bricks: border fluxes [nv][kCnsBorder] R | landing: FP32 [nv][S] f64, FP64 the second layer's [nv][S - S1] |
+//   neighbour slots [FP32: 2][2nd][256] u16
 template <class R, int ND>
 __host__ __device__ constexpr bool cns_land_in_prims() {
   return sizeof(R) == sizeof(double);
 }
 template <class R, int ND>
-__host__ __device__ constexpr size_t cns_layout_bytes(int hmax, int h1max) {
-  return 16 + (cns_land_in_prims<R, ND>() ? 8 * (size_t)(ND + 2) * (hmax - h1max) : 8 * (size_t)(ND + 2) * (kHaloTile + hmax)) +
-         sizeof(R) * (size_t)(2 * ND + 4 + ND * kCnsSlopeVars<ND>) * (kHaloTile + h1max) + 8 * (size_t)(ND + 2) * kHaloTile +
-         2 * 2 * (size_t)(2 * ND) * kHaloTile;
+__host__ __device__ constexpr size_t cns_layout_bytes(int hmax, int h1max, bool brick) {
+  const size_t rows = 2 * ND + 4 + ND * kCnsSlopeVars<ND>;
+  return 16 + 8 * (size_t)(ND + 2) * kHaloTile + sizeof(R) * rows * (kHaloTile + h1max) +
+         (brick ? sizeof(R) * (size_t)(ND + 2) * kCnsBorder<ND> : 0) +
+         (cns_land_in_prims<R, ND>() ? 8 * (size_t)(ND + 2) * (hmax - h1max) : 8 * (size_t)(ND + 2) * (kHaloTile + hmax)) +
+         (cns_land_in_prims<R, ND>() ? 1 : 2) * 2 * (size_t)(2 * ND) * kHaloTile;
 }
 
 #ifndef H3C_CNS_MINB
 #define H3C_CNS_MINB 2  // blocks per SM the CNS tile kernel is register-budgeted for
 #endif
 
-template <int ND, class R, int MODE, bool FUSE>
+// AUSM (euler/physics.hpp:276-293) with the splits' supersonic branches off
+// the common path: the same values as ausm (fv_kernels.cuh).
+template <class R, int ND>
+__device__ __forceinline__ void ausm_subsonic_first(const Prim<R, ND>& L, const Prim<R, ND>& Rt, int d, R* f) {
+  const R ML = L.M[d], MR = Rt.M[d];
+  const R tl = (ML + R(1)) * (ML + R(1)), tr = (MR + R(-1)) * (MR + R(-1));
+  R mi = R(0.25) * tl + R(-0.25) * tr;
+  R pl = (R(0.25) * tl) * (R(2) - ML), pr = (R(0.25) * tr) * (R(2) + MR);
+  if (beyond_one(ML) || beyond_one(MR)) {
+    mi = m_int<R>(R(1), ML) + m_int<R>(R(-1), MR);
+    pl = p_int<R>(R(1), ML);
+    pr = p_int<R>(R(-1), MR);
+  }
+  const R pi = pl * L.p + pr * Rt.p;
+  const bool left = mi >= R(0);
+  const R a = left ? L.a : Rt.a;
+#pragma unroll
+  for (int v = 0; v < ND + 1; ++v) f[v] = ((left ? L.q[v] : Rt.q[v]) * a) * mi;
+  f[ND + 1] = (((left ? L.q[ND + 1] + L.p : Rt.q[ND + 1] + Rt.p)) * a) * mi;
+#pragma unroll
+  for (int v = 0; v < ND; ++v)
+    if (v == d) f[v] = f[v] + pi;
+}
+
+// cell_dt of CNS (fv_kernels.cuh) in two parts.  On one level each part falls
+// as its argument grows, division by division, so the least time step of a
+// block is that of its largest wave speed S and largest viscous coefficient:
+// three divisions and a square root per cell, four more per block.
+template <int ND>
+__device__ __forceinline__ void cns_dt_args(const double* q, double h, const PhysConst& pc, double& S, double& coeff,
+                                            bool& bad) {
+  Prim<double, ND> P;
+#pragma unroll
+  for (int v = 0; v < ND + 2; ++v) P.q[v] = q[v];
+  make_prim<double, ND>(P, pc.gamma, pc.gm1);
+  bad = !(P.q[ND] > 0.0 && P.q[ND + 1] > 0.0 && P.p > 0.0);
+  S = -1.7976931348623157e308;
+#pragma unroll
+  for (int d = 0; d < ND; ++d) {
+    const double cand = fabs(P.u[d]) + P.a;
+    S = (S < cand) ? cand : S;
+  }
+  const double T = pc.gamma * P.p / P.q[ND];
+  coeff = sutherland<double>(T, pc.sOverTref, pc.sOverTrefP1) / (P.q[ND] * h);
+}
+__device__ __forceinline__ double cns_dt_of(double S, double coeff, double h, const PhysConst& pc) {
+  const double dt_inv = pc.cfl * h / S;
+  const double a1 = coeff / pc.Re0, a2 = coeff / (pc.Re0 * pc.Pr0 * pc.gm1);
+  const double S_visc = (a1 < a2) ? a2 : a1;
+  const double dt_v = pc.cflv * h / (2 * S_visc);
+  return (dt_v < dt_inv) ? dt_v : dt_inv;
+}
+
+// BRICK: constant row strides, and the minus faces on the tile's border come
+// from its list, evaluated before the direction loop by whole warps and
+// handed over through shared memory.  Left to their cells they are a sixth of
+// the tile's face evaluations, but in divergent branches of half the warps
+// and directions: 12 of a tile's 36 warp-wide evaluations, against 4 of 28.
+template <int ND, class R, int MODE, bool FUSE, bool BRICK>
 __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
     k_stage_cns_halo(const double* __restrict__ qin, double* out, Geometry g, CnsHaloGeom ch, PhysConst pc,
                      const Scalars* __restrict__ sc, long long* dtmin, int* status) {
@@ -105,15 +174,18 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
   constexpr int KH = kHaloMaxSlots / kHaloTile;
   constexpr bool LIP = cns_land_in_prims<R, ND>();
   const HaloGeom& hg = ch.h;
-  const int S = TB + hg.hmax, S1 = TB + ch.h1max, S2 = S - S1;
+  constexpr int NB = kCnsBorder<ND>;
+  const int S1 = BRICK ? TB + kCnsBrickH1<ND> : TB + ch.h1max;
+  const int S = TB + hg.hmax, S2 = S - TB - ch.h1max;
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem);
-  double* land = reinterpret_cast<double*>(smem + 16);                           // FP32: [NV][S]
-  R* pr = reinterpret_cast<R*>(land + (LIP ? 0 : (size_t)NV * S));              // [NPR][S1]
-  double* land2 = reinterpret_cast<double*>(pr + (size_t)NPR * S1);             // FP64: [NV][S2]
-  R* sl = reinterpret_cast<R*>(land2 + (LIP ? (size_t)NV * S2 : 0));             // [NSL][S1]
-  double* fx = reinterpret_cast<double*>(sl + (size_t)NSL * S1);                  // [NV][TB]
-  unsigned short* ln = reinterpret_cast<unsigned short*>(fx + NV * TB);           // [2][NP][TB]
+  double* fx = reinterpret_cast<double*>(smem + 16);                              // [NV][TB]
+  R* pr = reinterpret_cast<R*>(fx + NV * TB);                                     // [NPR][S1]
+  R* sl = pr + (size_t)NPR * S1;                                                  // [NSL][S1]
+  R* bm = sl + (size_t)NSL * S1;                                                  // [NV][NB]
+  double* land = reinterpret_cast<double*>(bm + (BRICK ? NV * NB : 0));           // FP32: [NV][S]
+  double* land2 = land;                                                           // FP64: [NV][S2]
+  unsigned short* ln = reinterpret_cast<unsigned short*>(land + (LIP ? (size_t)NV * S2 : (size_t)NV * S));  // [2][NP][TB]
   const int tid = threadIdx.x;
   const long long ld = g.ld;
   const R gamma = (R)pc.gamma, gm1 = (R)pc.gm1;
@@ -123,11 +195,12 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
 
   // where the state of slot s (tile, first or second layer) lands
   auto qslot = [&](int v, int s) -> double* {
-    if (LIP) return s < S1 ? reinterpret_cast<double*>(pr) + (size_t)v * S1 + s : land2 + (size_t)v * S2 + (s - S1);
+    if (LIP) return s < S1 ? reinterpret_cast<double*>(pr) + v * S1 + s : land2 + (size_t)v * S2 + (s - S1);
     return land + (size_t)v * S + s;
   };
 
   chain_begin();
+  const double k = sc->dt / h;  // single grids only
   long long tile = blockIdx.x;
   if (tile >= g.ntiles) return;
   if (tid == 0) {
@@ -213,7 +286,8 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
   };
   // the face flux F(l, r): AUSM + three-point viscous (cns/physics.hpp:155-161)
   auto face = [&](const Prim<R, ND>& L, const Prim<R, ND>& Rt, const R* sL, const R* sR, int d, R* f) {
-    ausm<R, ND>(L, Rt, d, f);
+    if (BRICK) ausm_subsonic_first<R, ND>(L, Rt, d, f);
+    else ausm<R, ND>(L, Rt, d, f);
     R fv[NV];
     viscous<R, ND>(L, Rt, sL, sR, d, hr, pc, fv);
 #pragma unroll
@@ -277,6 +351,9 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
         }
       }
     }
+    const unsigned bsel = BRICK && live ? __ldg(ch.bsel + c) : 0;  // per direction 1 + this cell's place in the list
+    unsigned entry = ~0u;
+    if (BRICK && tid < NB) entry = __ldg(ch.blist + tile * NB + tid);
     __syncthreads();  // primitives and slopes complete
 
     int hid_n[KH], o0_n = 0, nh1_n = 0, nh_n = 0;
@@ -284,6 +361,25 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
       if (next < g.ntiles) {
         nh_n = fetch_ids(next, hid_n, o0_n, nh1_n);
         issue(next, buf ^ 1, hid_n, nh_n);
+      }
+    }
+
+    // ---- bricks: the minus faces on the tile's border (a warp's entries share their direction) ----
+    if (BRICK && entry != ~0u) {
+      const int cs = entry & 0xff, m = (entry >> 8) & 0xfff, de = entry >> 20;
+#pragma unroll
+      for (int d = 0; d < ND; ++d) {
+        if (de != d) continue;
+        Prim<R, ND> Pc, Pn;
+        load_prim_s(cs, d, Pc);
+        load_prim_s(m, d, Pn);
+        R slc[ND * NV], sn[ND * NV];
+        load_slopes(cs, d, slc);
+        load_slopes(m, d, sn);
+        R f[NV];
+        face(Pn, Pc, sn, slc, d, f);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) bm[v * NB + tid] = f[v];
       }
     }
 
@@ -310,7 +406,11 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
       if (live) {
         const int m = L[(2 * d) * TB + tid];
         double fm[NV];
-        if (m < TB && L[(2 * d + 1) * TB + m] == tid) {
+        if (BRICK) {
+          const int b = (bsel >> (8 * d)) & 0xff;
+#pragma unroll
+          for (int v = 0; v < NV; ++v) fm[v] = b ? (double)bm[v * NB + b - 1] : fx[v * TB + m];
+        } else if (m < TB && L[(2 * d + 1) * TB + m] == tid) {
 #pragma unroll
           for (int v = 0; v < NV; ++v) fm[v] = fx[v * TB + m];
         } else {
@@ -333,11 +433,9 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
     }
 
     // ---- update and the next step's CFL minimum ----
-    long long ord = kOrdMax;
+    double S_max = -1.7976931348623157e308, coeff_max = S_max;
     bool bad = false;
     if (live) {
-      const double dt = sc[inst].dt;
-      const double k = dt / h;
       double qc[NV], qo[NV];  // FP32: the landing area already holds the next tile
 #pragma unroll
       for (int v = 0; v < NV; ++v) qc[v] = LIP ? *qslot(v, tid) : __ldg(qin + v * ld + c);
@@ -351,13 +449,25 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
 #pragma unroll
       for (int v = 0; v < NV; ++v) out[v * ld + c] = o[v];
       if (FUSE) {
-        const double cd = cell_dt<ND, CNS>(o, h, pc, nullptr, &bad);
-        if (!isnan(cd)) ord = dbl_to_ord(cd);
+        double wave, coeff;
+        cns_dt_args<ND>(o, h, pc, wave, coeff, bad);
+        if (wave > S_max) S_max = wave;  // a cell that is not finite (NaN) never wins
+        if (coeff > coeff_max) coeff_max = coeff;
       }
     }
     if (FUSE) {
       flag_bad_state(bad, sc, inst);
-      block_min_atomic(ord, per_instance(dtmin, inst));
+      // the warp's largest, its time step, then the block's least
+      for (int w = 16; w > 0; w >>= 1) {
+        S_max = fmax(S_max, __shfl_xor_sync(0xffffffffu, S_max, w));
+        coeff_max = fmax(coeff_max, __shfl_xor_sync(0xffffffffu, coeff_max, w));
+      }
+      long long ord = kOrdMax;
+      if ((tid & 31) == 0 && S_max > 0.0 && coeff_max > 0.0) {
+        const double cd = cns_dt_of(S_max, coeff_max, h, pc);
+        if (!isnan(cd)) ord = dbl_to_ord(cd);
+      }
+      block_min_atomic(ord, dtmin);
     }
     if (LIP) {  // FP64: the next tile lands where this one's primitives were
       __syncthreads();
@@ -382,9 +492,12 @@ bool halo_build_cns(int nd, long long ld, long long n_int, long long ntiles, con
                     const int* nbr, CnsHaloHost& H) {
   const int NP = 2 * nd, TB = kHaloTile;
   H.base.lnb.assign((size_t)NP * ld, 0);
+  const int NB = nd == 3 ? kCnsBorder<3> : kCnsBorder<2>, H1 = nd == 3 ? kCnsBrickH1<3> : kCnsBrickH1<2>;
   std::vector<std::vector<int>> l1s(ntiles), l2s(ntiles);
   std::vector<std::vector<unsigned short>> hns(ntiles);
-  std::atomic<bool> ok{true};
+  H.bsel.assign(ld, 0);
+  H.blist.assign((size_t)std::max<long long>(ntiles, 1) * NB, ~0u);
+  std::atomic<bool> ok{true}, brick{true};
   auto work = [&](long long t0, long long t1) {
     std::vector<int> l1, l2;
     std::vector<unsigned char> need;
@@ -441,6 +554,22 @@ bool halo_build_cns(int nd, long long ld, long long n_int, long long ntiles, con
       };
       for (long long c = c0; c < ce; ++c)
         for (int p = 0; p < NP; ++p) H.base.lnb[(size_t)p * ld + c] = slot(nbr[p * ld + c]);
+      // the border list (brick grids): minus faces that no plus face of the tile covers, whole warps per direction
+      int nb = 0;
+      for (int d = 0; d < nd && brick.load(std::memory_order_relaxed); ++d) {
+        nb = (nb + 31) / 32 * 32;
+        for (long long c = c0; c < ce; ++c) {
+          const long long v = nbr[(2 * d) * ld + c];
+          if (!outside(v) && nbr[(2 * d + 1) * ld + v] == c) continue;
+          if (nb >= NB || !outside(v)) {
+            brick = false;
+            break;
+          }
+          H.blist[(size_t)t * NB + nb] = (unsigned)(c - c0) | ((unsigned)slot(v) << 8) | ((unsigned)d << 20);
+          H.bsel[c] |= (unsigned)(nb + 1) << (8 * d);
+          ++nb;
+        }
+      }
       std::vector<unsigned short>& hn = hns[t];
       hn.assign(l1.size() * NP, 0xffff);
       for (size_t i = 0; i < l1.size(); ++i) {
@@ -487,19 +616,25 @@ bool halo_build_cns(int nd, long long ld, long long n_int, long long ntiles, con
   B.mean_halo = ntiles ? (double)nids / ntiles : 0.0;
   B.hmax = std::max(32, (mx + 31) / 32 * 32);
   H.h1max = std::max(32, (mx1 + 31) / 32 * 32);
+  H.brick = brick && H.h1max <= H1;
   return true;
 }
 
-size_t cns_halo_smem_bytes(int nd, bool mixed, int hmax, int h1max) {
-  if (nd == 2) return mixed ? cns_layout_bytes<float, 2>(hmax, h1max) : cns_layout_bytes<double, 2>(hmax, h1max);
-  return mixed ? cns_layout_bytes<float, 3>(hmax, h1max) : cns_layout_bytes<double, 3>(hmax, h1max);
+size_t cns_halo_smem_bytes(int nd, bool mixed, int hmax, int h1max, bool brick) {
+  if (brick) {  // rows as long as a brick's, the second layer's landing as wide as this grid's
+    const int h1 = nd == 3 ? kCnsBrickH1<3> : kCnsBrickH1<2>;
+    hmax += h1 - h1max;
+    h1max = h1;
+  }
+  if (nd == 2) return mixed ? cns_layout_bytes<float, 2>(hmax, h1max, brick) : cns_layout_bytes<double, 2>(hmax, h1max, brick);
+  return mixed ? cns_layout_bytes<float, 3>(hmax, h1max, brick) : cns_layout_bytes<double, 3>(hmax, h1max, brick);
 }
 
 namespace {
 
-template <int ND, class R, int MODE, bool FUSE>
+template <int ND, class R, int MODE, bool FUSE, bool BRICK>
 int cprep_one(size_t smem) {
-  auto k = k_stage_cns_halo<ND, R, MODE, FUSE>;
+  auto k = k_stage_cns_halo<ND, R, MODE, FUSE, BRICK>;
   // the opt-in limit (less the kernel's static arrays), not this grid's size: several solvers
   // share the kernel and its attribute
   int dev = 0, optin = 0;
@@ -519,44 +654,64 @@ int cprep_one(size_t smem) {
   }
   return nb;
 }
-template <int ND, class R, int MODE>
+template <int ND, class R, int MODE, bool BRICK>
 int cprep_f(size_t smem) {
-  return std::min(cprep_one<ND, R, MODE, false>(smem), cprep_one<ND, R, MODE, true>(smem));
+  return std::min(cprep_one<ND, R, MODE, false, BRICK>(smem), cprep_one<ND, R, MODE, true, BRICK>(smem));
+}
+template <int ND, class R, bool BRICK>
+int cprep_m(size_t smem) {
+  return std::min(std::min(cprep_f<ND, R, 0, BRICK>(smem), cprep_f<ND, R, 2, BRICK>(smem)),
+                  std::min(cprep_f<ND, R, 3, BRICK>(smem), cprep_f<ND, R, 4, BRICK>(smem)));
 }
 template <int ND, class R>
-int cprep_m(size_t smem) {
-  return std::min(std::min(cprep_f<ND, R, 0>(smem), cprep_f<ND, R, 2>(smem)),
-                  std::min(cprep_f<ND, R, 3>(smem), cprep_f<ND, R, 4>(smem)));
+int cprep(size_t smem, bool brick) {
+  return brick ? cprep_m<ND, R, true>(smem) : cprep_m<ND, R, false>(smem);
 }
 
-template <int ND, class R, int MODE>
-void claunch_f(bool fuse, const double* qin, double* out, const Geometry& g, const CnsHaloGeom& h,
-               const PhysConst& pc, const Scalars* sc, long long* dtmin, int* status, int grid, size_t smem,
-               cudaStream_t st) {
-  const auto k = fuse ? k_stage_cns_halo<ND, R, MODE, true> : k_stage_cns_halo<ND, R, MODE, false>;
+struct CnsLaunch {
+  const double* qin;
+  double* out;
+  const Geometry& g;
+  const CnsHaloGeom& h;
+  const PhysConst& pc;
+  const Scalars* sc;
+  long long* dtmin;
+  int* status;
+  int grid;
+  size_t smem;
+  cudaStream_t st;
+};
+template <int ND, class R, int MODE, bool FUSE>
+void claunch_b(const CnsLaunch& a) {
+  const auto k = a.h.blist ? k_stage_cns_halo<ND, R, MODE, FUSE, true> : k_stage_cns_halo<ND, R, MODE, FUSE, false>;
   // Chained (launch.hpp) where blocks take few tiles: 64^3 FP32 1141 -> 1106 us per 10 steps.  On long runs of
   // tiles per block the early start is worth nothing, and blocks that find an SM still taken by the kernel
   // before finish last (128^3, 28 tiles per block: 3205 -> 3245 us per 4 steps).
-  if (g.ntiles <= 8LL * grid) launch_chain(k, grid, kHaloTile, smem, st, qin, out, g, h, pc, sc, dtmin, status);
-  else k<<<grid, kHaloTile, smem, st>>>(qin, out, g, h, pc, sc, dtmin, status);
+  if (a.g.ntiles <= 8LL * a.grid)
+    launch_chain(k, a.grid, kHaloTile, a.smem, a.st, a.qin, a.out, a.g, a.h, a.pc, a.sc, a.dtmin, a.status);
+  else
+    k<<<a.grid, kHaloTile, a.smem, a.st>>>(a.qin, a.out, a.g, a.h, a.pc, a.sc, a.dtmin, a.status);
+}
+template <int ND, class R, int MODE>
+void claunch_f(bool fuse, const CnsLaunch& a) {
+  if (fuse) claunch_b<ND, R, MODE, true>(a);
+  else claunch_b<ND, R, MODE, false>(a);
 }
 template <int ND, class R>
-void claunch_m(int mode, bool fuse, const double* qin, double* out, const Geometry& g, const CnsHaloGeom& h,
-               const PhysConst& pc, const Scalars* sc, long long* dtmin, int* status, int grid, size_t smem,
-               cudaStream_t st) {
+void claunch_m(int mode, bool fuse, const CnsLaunch& a) {
   switch (mode) {
-    case 0: claunch_f<ND, R, 0>(fuse, qin, out, g, h, pc, sc, dtmin, status, grid, smem, st); break;
-    case 2: claunch_f<ND, R, 2>(fuse, qin, out, g, h, pc, sc, dtmin, status, grid, smem, st); break;
-    case 3: claunch_f<ND, R, 3>(fuse, qin, out, g, h, pc, sc, dtmin, status, grid, smem, st); break;
-    default: claunch_f<ND, R, 4>(fuse, qin, out, g, h, pc, sc, dtmin, status, grid, smem, st); break;
+    case 0: claunch_f<ND, R, 0>(fuse, a); break;
+    case 2: claunch_f<ND, R, 2>(fuse, a); break;
+    case 3: claunch_f<ND, R, 3>(fuse, a); break;
+    default: claunch_f<ND, R, 4>(fuse, a); break;
   }
 }
 
 }  // namespace
 
-int cns_halo_prepare(int nd, bool mixed, size_t smem) {
-  if (nd == 2) return mixed ? cprep_m<2, float>(smem) : cprep_m<2, double>(smem);
-  return mixed ? cprep_m<3, float>(smem) : cprep_m<3, double>(smem);
+int cns_halo_prepare(int nd, bool mixed, size_t smem, bool brick) {
+  if (nd == 2) return mixed ? cprep<2, float>(smem, brick) : cprep<2, double>(smem, brick);
+  return mixed ? cprep<3, float>(smem, brick) : cprep<3, double>(smem, brick);
 }
 
 void cns_halo_stage(int nd, bool mixed, int mode, bool fuse, const double* qin, double* out, const Geometry& g,
@@ -566,12 +721,13 @@ void cns_halo_stage(int nd, bool mixed, int mode, bool fuse, const double* qin, 
     const unsigned nb = (unsigned)((gt.ng + kBlock - 1) / kBlock);
     launch_chain(nd == 2 ? k_ghost_slopes<2> : k_ghost_slopes<3>, nb, kBlock, 0, st, qin, g, gt, gsl, h.ngl);
   }
+  const CnsLaunch a{qin, out, g, h, pc, sc, dtmin, status, grid, smem, st};
   if (nd == 2) {
-    if (mixed) claunch_m<2, float>(mode, fuse, qin, out, g, h, pc, sc, dtmin, status, grid, smem, st);
-    else claunch_m<2, double>(mode, fuse, qin, out, g, h, pc, sc, dtmin, status, grid, smem, st);
+    if (mixed) claunch_m<2, float>(mode, fuse, a);
+    else claunch_m<2, double>(mode, fuse, a);
   } else {
-    if (mixed) claunch_m<3, float>(mode, fuse, qin, out, g, h, pc, sc, dtmin, status, grid, smem, st);
-    else claunch_m<3, double>(mode, fuse, qin, out, g, h, pc, sc, dtmin, status, grid, smem, st);
+    if (mixed) claunch_m<3, float>(mode, fuse, a);
+    else claunch_m<3, double>(mode, fuse, a);
   }
 }
 

@@ -91,10 +91,6 @@ __device__ __forceinline__ double* at32(double* row, unsigned c) {
   return reinterpret_cast<double*>(reinterpret_cast<char*>(row) + c * 8u);
 }
 
-// |M| >= 1 or NaN, from the exponent bits (at exactly 1 the subsonic and supersonic splits agree)
-__device__ __forceinline__ bool beyond_one(double M) { return (__double2hiint(M) & 0x7fffffff) >= 0x3ff00000; }
-__device__ __forceinline__ bool beyond_one(float M) { return (__float_as_int(M) & 0x7fffffff) >= 0x3f800000; }
-
 // a load the compiler may not move ahead of the phase before it (its registers are needed there)
 __device__ __forceinline__ uint4 load_here(const uint4* p) {
   uint4 r;

@@ -99,6 +99,10 @@ struct CnsHaloGeom {
   const double* __restrict__ gsl;            // [nd * nv][ngl] slopes of the ghost cells
   long long ngl;                             // leading dimension of gsl
   int h1max;                                 // layer-1 slots reserved per tile (multiple of 32)
+  // brick grids (else nullptr): per tile the minus faces on its border -- cell slot, neighbour slot << 8,
+  // direction << 20, all ones where padded -- and per cell, 8 bits per direction, 1 + its entry (0: none)
+  const unsigned* __restrict__ blist;
+  const unsigned* __restrict__ bsel;
 };
 
 struct CnsHaloHost {
@@ -106,12 +110,14 @@ struct CnsHaloHost {
   std::vector<int> h1end;
   std::vector<unsigned short> hnb;
   int h1max = 0;
+  bool brick = false;                        // every tile fits the brick variant (h3c_stage_cns.cu)
+  std::vector<unsigned> blist, bsel;
 };
 
 bool halo_build_cns(int nd, long long ld, long long n_int, long long ntiles, const std::vector<long long>& tile_end,
                     const int* nbr, CnsHaloHost& H);
-size_t cns_halo_smem_bytes(int nd, bool mixed, int hmax, int h1max);
-int cns_halo_prepare(int nd, bool mixed, size_t smem);
+size_t cns_halo_smem_bytes(int nd, bool mixed, int hmax, int h1max, bool brick);
+int cns_halo_prepare(int nd, bool mixed, size_t smem, bool brick);
 // the ghost-slope pass and the stage; h = the grid's (single) cell length
 void cns_halo_stage(int nd, bool mixed, int mode, bool fuse, const double* qin, double* out, const Geometry& g,
                     const GhostTables& gt, const CnsHaloGeom& h, const PhysConst& pc, const Scalars* sc,
