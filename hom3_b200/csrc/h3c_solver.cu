@@ -511,15 +511,15 @@ void stage_t(h3c_solver s, const double* qin, double* out) {
 // Euler adjoint stage in the tile kernel (one block per Morton tile)
 template <int ND, bool HANG>
 static void adj_ausm_t(h3c_solver s, const double* qin, const double* lamin, double* gout, const double* extra,
-                       const double* extra2, double alpha, double beta, double gam, double gam2) {
+                       const double* extra2, double alpha, double beta, double gam, double gam2, const double* dt) {
   constexpr size_t smem = adj_ausm_smem_bytes<ND>();
   static bool attr = false;  // one opt-in per instantiation (dynamic smem above 48 KB)
   if (!attr) {
     cudaFuncSetAttribute(k_adj_ausm<ND, HANG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     attr = true;
   }
-  k_adj_ausm<ND, HANG><<<(unsigned)std::max<long long>(1, s->ntiles), kBlock, smem, s->stream>>>(
-      qin, lamin, gout, extra, extra2, alpha, beta, gam, gam2, geometry(s), ghosts(s), s->pc, s->d_sc);
+  launch_chain(k_adj_ausm<ND, HANG>, (unsigned)std::max<long long>(1, s->ntiles), kBlock, smem, s->stream, qin, lamin,
+               gout, extra, extra2, alpha, beta, gam, gam2, geometry(s), ghosts(s), s->pc, dt);
 }
 
 template <int ND, int PHYS, int FLUX, class R, int MODE, bool HANG>
@@ -2433,6 +2433,9 @@ int h3c_adjoint(h3c_solver s, int64_t nsteps, int64_t every, const double* dJ_dq
   double* lamD = lam + 3 * Q;  // first-stage output cotangent (SSP-RK3)
   cudaMemsetAsync(lam, 0, sizeof(double) * Q * 4, s->stream);
   if (int rc = caller_to_internal(s, dJ_dqN, lamA)) return rc;
+  // the Euler tile adjoint reads the step's dt where the forward run recorded it, the others from the scalars
+  const bool adj_tile = s->desc.physics == H3C_EULER && s->desc.flux == H3C_FLUX_AUSM && !muscl && s->tile;
+  const double* dt_now = d_dts;
   auto adj = [&](const double* qin, const double* lamin, double* gout, double alpha, double beta,
                  const double* extra = nullptr, double gam = 0.0, const double* extra2 = nullptr,
                  double gam2 = 0.0) {
@@ -2488,11 +2491,11 @@ int h3c_adjoint(h3c_solver s, int64_t nsteps, int64_t every, const double* dJ_dq
     }
     if (s->desc.physics == H3C_EULER && s->tile) {
       if (s->nd == 2) {
-        if (s->nsub > 0) adj_ausm_t<2, true>(s, qin, lamin, gout, extra, extra2, alpha, beta, gam, gam2);
-        else adj_ausm_t<2, false>(s, qin, lamin, gout, extra, extra2, alpha, beta, gam, gam2);
+        if (s->nsub > 0) adj_ausm_t<2, true>(s, qin, lamin, gout, extra, extra2, alpha, beta, gam, gam2, dt_now);
+        else adj_ausm_t<2, false>(s, qin, lamin, gout, extra, extra2, alpha, beta, gam, gam2, dt_now);
       } else {
-        if (s->nsub > 0) adj_ausm_t<3, true>(s, qin, lamin, gout, extra, extra2, alpha, beta, gam, gam2);
-        else adj_ausm_t<3, false>(s, qin, lamin, gout, extra, extra2, alpha, beta, gam, gam2);
+        if (s->nsub > 0) adj_ausm_t<3, true>(s, qin, lamin, gout, extra, extra2, alpha, beta, gam, gam2, dt_now);
+        else adj_ausm_t<3, false>(s, qin, lamin, gout, extra, extra2, alpha, beta, gam, gam2, dt_now);
       }
       return;
     }
@@ -2525,7 +2528,8 @@ int h3c_adjoint(h3c_solver s, int64_t nsteps, int64_t every, const double* dJ_dq
     }
     for (long long i = i1 - 1; i >= i0; --i) {
       double* s0 = seg + Q * per * (i - i0);
-      {
+      dt_now = d_dts + i;
+      if (!adj_tile) {
         Launch L3(s, K_SCALAR);
         k_set_dt_from<<<1, 1, 0, s->stream>>>(s->d_sc, d_dts, i);
       }
