@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kHaloTile, split_minb<ND, R>())
     }
     __syncthreads();
 
-    // ---- faces: AUSM flux (physics.hpp:276-293) from both sides' splits and pressures and the upwind theta ----
+    // ---- faces: AUSM flux (euler/physics.hpp:276-293) from both sides' splits and pressures and the upwind theta ----
     auto pressure_sum = [&](P2 l, P2 r, R pl, R pr) -> R {
       if (F32) return (R)fmaf((float)l.y, (float)pl, __fmul_rn((float)r.y, (float)pr));
       return l.y + r.y;
