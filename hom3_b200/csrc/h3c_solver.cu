@@ -392,14 +392,21 @@ void launch_slopes_ptr(h3c_solver s, const double* q) {
 
 void launch_slopes(h3c_solver s, int which) { launch_slopes_ptr(s, s->d_q[which]); }
 
+// Two threads per cell in the 2D MUSCL kernels (muscl_kernels.cuh) up to one
+// block of them per SM.  SSP-RK3, 30 steps, us with one / two threads: 64^2
+// 1145 / 911, 128^2 1164 / 976, 256^2 1431 / 1684, 400^2 2809 / 2969.
+bool muscl_split(h3c_solver s) { return s->nd == 2 && s->n_int <= (long long)kBlock / 2 * num_sms(); }
+
 // EXTENSION: limited least-squares gradients of the stage input (MUSCL)
 // ghosts_too: the periodic ghosts' copies as well (the adjoint reads them; the stage reads through d_gsrc)
 void launch_grad(h3c_solver s, const double* q, bool ghosts_too) {
   Launch L(s, K_SLOPES);
   const double K = s->desc.limiter_k;
-  const auto grad = s->nd == 2 ? (s->nsub > 0 ? k_muscl_grad<2, true> : k_muscl_grad<2, false>)
-                               : (s->nsub > 0 ? k_muscl_grad<3, true> : k_muscl_grad<3, false>);
-  launch_chain(grad, blocks(s->n_int), kBlock, 0, s->stream, q, s->d_xc, geometry(s), s->pc, K, s->d_slopes);
+  const bool two = muscl_split(s);
+  const auto grad = s->nd == 2 ? (s->nsub > 0 ? (two ? k_muscl_grad<2, true, 2> : k_muscl_grad<2, true, 1>)
+                                              : (two ? k_muscl_grad<2, false, 2> : k_muscl_grad<2, false, 1>))
+                               : (s->nsub > 0 ? k_muscl_grad<3, true, 1> : k_muscl_grad<3, false, 1>);
+  launch_chain(grad, blocks(two ? 2 * s->n_int : s->n_int), kBlock, 0, s->stream, q, s->d_xc, geometry(s), s->pc, K, s->d_slopes);
   if (ghosts_too && s->needs_periodic) {
     if (s->nd == 2) k_muscl_ghosts<2><<<blocks(s->ng), kBlock, 0, s->stream>>>(s->d_slopes, geometry(s), ghosts(s));
     else k_muscl_ghosts<3><<<blocks(s->ng), kBlock, 0, s->stream>>>(s->d_slopes, geometry(s), ghosts(s));
@@ -410,8 +417,10 @@ template <int ND, int PHYS, int FLUX, class R, int MODE, bool HANG, bool FUSE>
 void stage_t(h3c_solver s, const double* qin, double* out) {
   Launch L(s, MODE == 0 ? K_STAGE1 : K_STAGE2);
   if (PHYS == EULER && FLUX == AUSM && s->desc.reconstruction == H3C_RECON_MUSCL) {
-    launch_chain(k_stage_muscl<ND, R, MODE, HANG, FUSE>, blocks(s->n_int), kBlock, 0, s->stream, qin, out, s->d_slopes,
-                 s->d_xc, geometry(s), s->pc, s->d_sc, &s->d_sc->dtmin_ord, s->needs_periodic ? s->d_gsrc : nullptr);
+    const bool two = ND == 2 && muscl_split(s);
+    launch_chain(two ? k_stage_muscl<ND, R, MODE, HANG, FUSE, ND == 2 ? 2 : 1> : k_stage_muscl<ND, R, MODE, HANG, FUSE, 1>,
+                 blocks(two ? 2 * s->n_int : s->n_int), kBlock, 0, s->stream, qin, out, s->d_slopes, s->d_xc, geometry(s),
+                 s->pc, s->d_sc, &s->d_sc->dtmin_ord, s->needs_periodic ? s->d_gsrc : nullptr);
     return;
   }
   if (PHYS == CNS && s->tile && s->halo && s->cns_ok) {

@@ -73,31 +73,49 @@ __device__ __forceinline__ double vk_phi(double a, double b, double e2) {
   return ((a * a + e2) * b + 2. * b * b * a) * nr_rcp(b * (a * a + 2. * b * b + a * b + e2));
 }
 
-template <int ND, bool HANG>
+// The cell a thread of a split kernel works on and its share of it: SPLIT
+// threads per cell, in different warps of the block.
+template <int SPLIT> __device__ __forceinline__ long long split_cell(int& sub) {
+  constexpr int TC = kBlock / SPLIT;  // cells per block
+  sub = SPLIT == 1 ? 0 : threadIdx.x / TC;
+  return (long long)blockIdx.x * TC + (SPLIT == 1 ? threadIdx.x : threadIdx.x % TC);
+}
+
+// SPLIT 2 (2D): two threads per cell, each with half of the variables.  Small
+// grids have too few cells to hide a thread's chain of a thousand dependent
+// instructions: 256^2 cells are 3.5 warps per scheduler, of which the FP64
+// pipe sees a third.
+template <int ND, bool HANG, int SPLIT>
 __global__ void __launch_bounds__(kBlock) k_muscl_grad(const double* __restrict__ q, const double* __restrict__ xc,
                                                        Geometry g, PhysConst pc, double limiter_k,
                                                        double* __restrict__ grad) {
   constexpr int NV = ND + 2;
+  constexpr int NL = NV / SPLIT;  // this thread's variables: sub * NL ...
   chain_begin();
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= instance_end(g, tile_instance(g, blockIdx.x))) return;  // also skips padding between instances
+  int sub;
+  const long long c = split_cell<SPLIT>(sub);
+  if (c >= g.n_int || c >= instance_end(g, tile_instance(g, c / kBlock))) return;  // also skips padding between instances
+  auto own = [&](const double* w, int v) { return SPLIT == 1 || sub == 0 ? w[v] : w[v + NV - NL]; };
   const long long ld = g.ld;
   const double gm1 = pc.gm1;
-  double wc[NV], wmax[NV], wmin[NV];
-  prim_w<ND>(q, ld, c, gm1, wc);
+  double wc[NL], wmax[NL], wmin[NL];
+  {
+    double w[NV];
+    prim_w<ND>(q, ld, c, gm1, w);
 #pragma unroll
-  for (int v = 0; v < NV; ++v) { wmax[v] = wc[v]; wmin[v] = wc[v]; }
+    for (int v = 0; v < NL; ++v) { wc[v] = own(w, v); wmax[v] = wc[v]; wmin[v] = wc[v]; }
+  }
   double xcc[ND];
 #pragma unroll
   for (int k = 0; k < ND; ++k) xcc[k] = __ldg(xc + k * ld + c);
-  double M[ND][ND], b[NV][ND];
+  double M[ND][ND], b[NL][ND];
 #pragma unroll
   for (int i = 0; i < ND; ++i) {
 #pragma unroll
     for (int j = 0; j < ND; ++j) M[i][j] = 0.0;
   }
 #pragma unroll
-  for (int v = 0; v < NV; ++v) {
+  for (int v = 0; v < NL; ++v) {
 #pragma unroll
     for (int i = 0; i < ND; ++i) b[v][i] = 0.0;
   }
@@ -118,12 +136,12 @@ __global__ void __launch_bounds__(kBlock) k_muscl_grad(const double* __restrict_
       for (int j = 0; j < ND; ++j) M[i][j] = M[i][j] + (wgt * dx[i]) * dx[j];
     }
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const double dw = wn[v] - wc[v];
+    for (int v = 0; v < NL; ++v) {
+      const double wv = own(wn, v), dw = wv - wc[v];
 #pragma unroll
       for (int i = 0; i < ND; ++i) b[v][i] = b[v][i] + (wgt * dx[i]) * dw;
-      wmax[v] = wn[v] > wmax[v] ? wn[v] : wmax[v];
-      wmin[v] = wn[v] < wmin[v] ? wn[v] : wmin[v];
+      wmax[v] = wv > wmax[v] ? wv : wmax[v];
+      wmin[v] = wv < wmin[v] ? wv : wmin[v];
     }
   });
   double inv[ND][ND];
@@ -151,9 +169,9 @@ __global__ void __launch_bounds__(kBlock) k_muscl_grad(const double* __restrict_
   }
   const double kh = limiter_k * g.len[g.lvl[c]];
   const double e2 = kh * kh * kh;
-  double G[NV][ND], psi[NV];
+  double G[NL][ND], psi[NL];
 #pragma unroll
-  for (int v = 0; v < NV; ++v) {
+  for (int v = 0; v < NL; ++v) {
 #pragma unroll
     for (int i = 0; i < ND; ++i) {
       double s = inv[i][0] * b[v][0];
@@ -173,7 +191,7 @@ __global__ void __launch_bounds__(kBlock) k_muscl_grad(const double* __restrict_
 #pragma unroll
     for (int k = 0; k < ND; ++k) xf[k] = xf[k] - xcc[k];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
+    for (int v = 0; v < NL; ++v) {
       double d2 = G[v][0] * xf[0];
 #pragma unroll
       for (int k = 1; k < ND; ++k) d2 = d2 + G[v][k] * xf[k];
@@ -184,9 +202,9 @@ __global__ void __launch_bounds__(kBlock) k_muscl_grad(const double* __restrict_
     }
   });
 #pragma unroll
-  for (int v = 0; v < NV; ++v) {
+  for (int v = 0; v < NL; ++v) {
 #pragma unroll
-    for (int i = 0; i < ND; ++i) grad[(v * ND + i) * ld + c] = psi[v] * G[v][i];
+    for (int i = 0; i < ND; ++i) grad[((sub * NL + v) * ND + i) * ld + c] = psi[v] * G[v][i];
   }
 }
 
@@ -224,26 +242,35 @@ __device__ __forceinline__ void prim_from_w(const double* w, R gamma, R igm1, Pr
   for (int d = 0; d < ND; ++d) P.M[d] = P.u[d] * ainv;
 }
 
-template <int ND, class R, int MODE, bool HANG, bool FUSE>
+// SPLIT 2 (2D): the two directions of a cell by two threads; the second's sum
+// goes to the first through shared memory.
+template <int ND, class R, int MODE, bool HANG, bool FUSE, int SPLIT>
 __global__ void __launch_bounds__(kBlock) k_stage_muscl(const double* __restrict__ qin, double* out,
                                                         const double* __restrict__ grad,
                                                         const double* __restrict__ xc, Geometry g, PhysConst pc,
                                                         const Scalars* __restrict__ sc, long long* dtmin,
                                                         const int* __restrict__ gsrc) {
   constexpr int NV = ND + 2;
+  static_assert(SPLIT == 1 || SPLIT == ND, "a thread per cell, or per cell and direction");
+  __shared__ double sacc[SPLIT > 1 ? NV : 1][SPLIT > 1 ? kBlock / SPLIT : 1];
   chain_begin();
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int inst = tile_instance(g, blockIdx.x);
-  const bool live = c < instance_end(g, inst);
+  int sub;
+  const long long c = split_cell<SPLIT>(sub);
+  const int inst = c < g.n_int ? tile_instance(g, c / kBlock) : 0;
+  bool live = c < g.n_int && c < instance_end(g, inst);
+  const long long ld = g.ld;
+  double acc[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) acc[v] = 0.0;
   long long ord = kOrdMax;
   bool bad = false;
+  double dt = 0.0, dx = 1.0, qc[NV];
   if (live) {
-    const long long ld = g.ld;
-    const double dt = sc[inst].dt;
-    const double dx = g.len[g.lvl[c]];
+    dt = sc[inst].dt;
+    dx = g.len[g.lvl[c]];
     const double gm1 = pc.gm1;
     const R gamma = (R)pc.gamma, igm1 = R(1) / (R)pc.gm1;
-    double qc[NV], wc[NV], Gc[NV * ND], xcc[ND];
+    double wc[NV], Gc[NV * ND], xcc[ND];
 #pragma unroll
     for (int v = 0; v < NV; ++v) qc[v] = __ldg(qin + v * ld + c);
     prim_w<ND>(qin, ld, c, gm1, wc);
@@ -251,9 +278,6 @@ __global__ void __launch_bounds__(kBlock) k_stage_muscl(const double* __restrict
     for (int k = 0; k < NV * ND; ++k) Gc[k] = __ldg(grad + k * ld + c);
 #pragma unroll
     for (int k = 0; k < ND; ++k) xcc[k] = __ldg(xc + k * ld + c);
-    double acc[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) acc[v] = 0.0;
     // flux of the face between c and n along d (side: where n lies), into f
     auto face = [&](int n, int d, int side, double* fo) {
       const int L = side < 0 ? n : (int)c, Rr = side < 0 ? (int)c : n;
@@ -309,12 +333,28 @@ __global__ void __launch_bounds__(kBlock) k_stage_muscl(const double* __restrict
     };
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
+      if (SPLIT > 1 && d != sub) continue;  // the same for a whole warp
       double fm[NV], fp[NV];
       side_flux(g.nbr[(2 * d) * ld + c], d, -1, fm);
       side_flux(g.nbr[(2 * d + 1) * ld + c], d, 1, fp);
 #pragma unroll
       for (int v = 0; v < NV; ++v) acc[v] = acc[v] + (fm[v] - fp[v]);
     }
+  }
+  if (SPLIT > 1) {
+    constexpr int TC = kBlock / SPLIT;
+    if (sub > 0) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v) sacc[v][threadIdx.x % TC] = acc[v];
+    }
+    __syncthreads();
+    live = live && sub == 0;  // one thread updates the cell
+    if (live) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v) acc[v] = acc[v] + sacc[v][threadIdx.x];
+    }
+  }
+  if (live) {
     const double k = dt / dx;
     double o[NV];
 #pragma unroll
