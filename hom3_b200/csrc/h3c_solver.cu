@@ -118,7 +118,7 @@ struct h3c_solver_s {
   bool tile = true;  // Euler stages use the shared-memory tile kernel
   bool cns_adj_dual = false;  // CNS adjoint faces by dual numbers instead of the hand-written reverse
   int halo_cap = 0;           // cap on the Euler halo entries held in shared memory (0: none)
-  int euler_kernel = 1;       // Euler/AUSM stage: 0 halo-staged tile, 1 per-lane tile, 2 per cell, 3 warp-tiled,
+  int euler_kernel = 1;       // Euler/AUSM stage: 0 halo-staged tile, 1 split tile, 2 per cell, 3 warp-tiled,
                               // 4 per-lane tile of 512 cells (3D, one grid)
   int warp_bps = 0;           // resident blocks per SM of the warp-tiled kernel (0: unavailable)
   // halo-staged Euler/AUSM stage (h3c_stage_halo.cu): tables, launch size
@@ -2157,7 +2157,7 @@ struct TuneCand {
   int persist;
 };
 constexpr TuneCand kTune[] = {
-    {true, 1, 0}, {true, 1, 1}, {true, 1, 2}, {true, 1, 3}, {true, 1, 4},  // per-lane tile (CNS: its tile kernel)
+    {true, 1, 0}, {true, 1, 1}, {true, 1, 2}, {true, 1, 3}, {true, 1, 4},  // split tile (CNS: its tile kernel)
     {false, 2, 0},                                                          // generic per-cell kernels
     {true, 2, 0},                                                           // per-cell AUSM kernel
     {true, 0, 1}, {true, 0, 2}, {true, 0, 3},                               // halo-staged tile kernel

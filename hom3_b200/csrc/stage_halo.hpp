@@ -57,7 +57,7 @@ struct HaloHost {
 // (>= 0 cell, <= -2 sub-face group -2 - k of sub [2^(nd-1)][nsub]) for the
 // tiles of [0, n_int); tile_end[t] is the end of tile t's cells (tiles never
 // span two batch instances).  Returns false when a tile's slots overflow 15
-// bits or the cells 29 bits (the caller then keeps the per-lane tile kernel).
+// bits or the cells 29 bits (the caller then takes the per-lane tile kernel).
 // Halo ids carry the direction in bits 29-30, the side in bit 31.
 bool halo_build(int nd, long long ld, long long ntiles, const std::vector<long long>& tile_end, const int* nbr,
                 const int* sub, long long nsub, HaloHost& H);

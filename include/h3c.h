@@ -201,7 +201,7 @@ int h3c_instances(h3c_solver s, double* dt, double* time, int64_t* step);
  * solver, from the same saved state, restores the state and keeps the
  * fastest (sets H3C_OPT_TILE_KERNEL, H3C_OPT_EULER_KERNEL and
  * H3C_OPT_PERSISTENT_BLOCKS); returns its index and its time per step (ms).
- * Index: 0-4 the per-lane tile kernel (CNS: the CNS tile kernel) with its
+ * Index: 0-4 the split tile kernel (CNS: the CNS tile kernel) with its
  * default grid or 1-4 persistent blocks per SM; 5 the generic per-cell
  * kernels; 6 the per-cell AUSM kernel; 7-9 the halo-staged tile kernel with
  * 1-3 persistent blocks per SM; 10 the warp-tiled kernel. */
@@ -309,12 +309,12 @@ int h3c_launches(h3c_solver s, int64_t* n);
  * H3C_OPT_GRAPHS       replay runs of steps from a captured CUDA graph (default 1)
  * H3C_OPT_HALO_KERNEL  the halo-staged tile kernels (each tile and its halo copied into shared
  *                      memory by bulk copies) may be used: the CNS stage and H3C_OPT_EULER_KERNEL 0
- *                      (default 1; 0: CNS steps in the per-cell kernel, Euler kernel 0 in the per-lane one) */
+ *                      (default 1; 0: CNS steps in the per-cell kernel, Euler kernel 0 in the split one) */
 #define H3C_OPT_TILE_KERNEL 1
 #define H3C_OPT_GRAPHS 2
 #define H3C_OPT_HALO_KERNEL 3
 /* H3C_OPT_PERSISTENT_BLOCKS  blocks of the Euler/AUSM stage launch, each looping over tiles
- *                            (0, the default: one block per tile for the per-lane tile kernel,
+ *                            (0, the default: one block per tile for the split tile kernel,
  *                            the resident blocks of all SMs for the halo-staged one) */
 #define H3C_OPT_PERSISTENT_BLOCKS 4
 /* H3C_OPT_CNS_ADJOINT_DUAL  the CNS adjoint's face derivatives by forward-mode dual numbers instead
@@ -325,7 +325,8 @@ int h3c_launches(h3c_solver s, int64_t* n);
  *                     are read from global memory where a face needs them */
 #define H3C_OPT_HALO_SLOTS 6
 /* H3C_OPT_EULER_KERNEL  the Euler/AUSM stage kernel (with the tile kernels on): 0 the halo-staged
- *                       tile kernel when its tables exist, 1 (the default) the per-lane tile kernel,
+ *                       tile kernel when its tables exist, 1 (the default) the split tile kernel
+ *                       (flux splits once per cell; grids beyond its tables' indices: the per-lane one),
  *                       2 one thread per cell, faces from both sides, 3 one warp per 32 Morton cells
  *                       (each face state once per warp, each face between two of its cells once),
  *                       4 the per-lane tile kernel on 512-cell tiles (8x8x8 Morton bricks, 512-thread
@@ -333,7 +334,7 @@ int h3c_launches(h3c_solver s, int64_t* n);
 #define H3C_OPT_EULER_KERNEL 7
 int h3c_set_option(h3c_solver s, int option, int value);
 /* The Euler stage launch in use (no hom3 counterpart): info[0] kernel (0 per
- * cell, 1 per-lane tile, 2 halo-staged tile, 3 the per-cell AUSM kernel, 4 the warp-tiled AUSM
+ * cell, 1 split tile, 2 halo-staged tile, 3 the per-cell AUSM kernel, 4 the warp-tiled AUSM
  * kernel, 5 the per-lane tile kernel on 512-cell tiles), [1] halo slots per tile, [2]
  * largest tile halo, [3] mean tile halo x 1000, [4] resident blocks per SM
  * of the halo-staged kernel, [5] blocks launched, [6] its dynamic shared
