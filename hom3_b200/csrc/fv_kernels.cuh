@@ -210,6 +210,24 @@ __device__ __forceinline__ void flag_timeout(const Scalars* sc, int* status) {
 // StepBegin: 256^2 MUSCL, SSP-RK3, 30 steps 2187 -> 1465 us; 48 coupled
 // 512 x 192 steps 2458 -> 1481 us).  Every kernel launched that way starts
 // with this call.
+// The set-up tables do not change while kernels run, so what a block needs of
+// them first (a cell's neighbours, a ghost's boundary cell) is loaded before
+// the wait, by load_here: a load the compiler keeps where it stands.
+__device__ __forceinline__ int load_here(const int* p) {
+  int r;
+  asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(r) : "l"(p) : "memory");
+  return r;
+}
+__device__ __forceinline__ int load_here(const unsigned char* p) {
+  unsigned r;
+  asm volatile("ld.global.nc.u8 %0, [%1];" : "=r"(r) : "l"(p) : "memory");
+  return (int)r;
+}
+__device__ __forceinline__ uint4 load_here(const uint4* p) {
+  uint4 r;
+  asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+  return r;
+}
 __device__ __forceinline__ void chain_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
@@ -651,29 +669,29 @@ __global__ void __launch_bounds__(kBlock) k_bc(double* __restrict__ q, const dou
                                                Geometry g, GhostTables gt, PhysConst pc,
                                                const Scalars* sc, PartnerView pv, StepBegin begin) {
   constexpr int NV = nvars<ND, PHYS>();
-  chain_begin();
-  unsigned blk = blockIdx.x;
-  if (begin.sc) {  // the first block does the step's scalar work; no condition launched with it reads the scalars
-    if (blk == 0) {
-      step_begin(begin);
-      return;
-    }
-    --blk;
-  }
+  const unsigned blk = blockIdx.x - (begin.sc ? 1 : 0);  // with scalar work, the first block does that
   const long long i = (long long)blk * blockDim.x + threadIdx.x;
-  if (i >= gt.ng) return;
-  const int b = gt.bc_apply[i];
-  if (b == 255) return;
+  const bool ghost = !(begin.sc && blockIdx.x == 0) && i < gt.ng;
+  int b = 255, bc = 0, kind = BC_EXCHANGE;
+  if (ghost) {
+    b = load_here(gt.bc_apply + i);
+    bc = load_here(gt.bndry + i);
+    if (b != 255) kind = load_here(&gt.bcs[b].kind);
+  }
+  chain_begin();
+  if (begin.sc && blockIdx.x == 0) {  // no condition launched with it reads the scalars
+    step_begin(begin);
+    return;
+  }
+  if (b == 255 || kind == BC_EXCHANGE) return;  // no condition, or written by the caller (another solver's cells)
   const BcParam& B = gt.bcs[b];
-  if (B.kind == BC_EXCHANGE) return;  // written by the caller (another solver's cells)
   const long long gcell = g.n_int + i;
-  const int bc = gt.bndry[i];
   const long long ld = g.ld;
   double qb[NV];
 #pragma unroll
   for (int v = 0; v < NV; ++v) qb[v] = q[v * ld + bc];
   double out[NV];
-  switch (B.kind) {
+  switch (kind) {
     case BC_EULER_NEUMANN:  // euler/boundary_conditions.hpp:17-43
     case BC_HEAT_NEUMANN:   // heat/boundary_conditions.hpp:40-63
 #pragma unroll
@@ -732,8 +750,8 @@ __global__ void __launch_bounds__(kBlock) k_bc(double* __restrict__ q, const dou
       if (gt.partner[i] < 0 || pv.q == nullptr) return;
       const double Tother = partner_T(B, pv, gt.partner[i]);
       const double Tthis = qlhs[bc];
-      const double kap = B.kind == BC_CPL_HEAT_CNS ? B.v[0] : 0.0;  // EXTENSION: k_solid / k_fluid
-      const double Ts = B.kind == BC_CPL_HEAT_CNS
+      const double kap = kind == BC_CPL_HEAT_CNS ? B.v[0] : 0.0;  // EXTENSION: k_solid / k_fluid
+      const double Ts = kind == BC_CPL_HEAT_CNS
                             ? ((kap == 0.0 || kap == 1.0) ? 0.5 * (Tother + Tthis) : (Tother + kap * Tthis) / (1.0 + kap))
                             : 0.5 * (Tthis + Tother);
       out[0] = 2.0 * Ts - qb[0];
@@ -754,23 +772,23 @@ __global__ void __launch_bounds__(kBlock) k_bc(double* __restrict__ q, const dou
       bp[ND + 1] = (gamma - 1.0) * (qb[ND + 1] - 0.5 * qb[ND] * vm2);
 #pragma unroll
       for (int v = 0; v < ND + 2; ++v) gp[v] = bp[v];
-      if (B.kind == BC_CNS_INFLOW) {  // cns/boundary_conditions.hpp:37-61
+      if (kind == BC_CNS_INFLOW) {  // cns/boundary_conditions.hpp:37-61
 #pragma unroll
         for (int d = 0; d < ND; ++d) gp[d] = 2.0 * B.v[d] - bp[d];
         gp[ND] = 2.0 * B.v[ND] - bp[ND];
-      } else if (B.kind == BC_CNS_OUTFLOW) {  // :81-101
+      } else if (kind == BC_CNS_OUTFLOW) {  // :81-101
         gp[ND + 1] = 2.0 * B.v[ND + 1] - bp[ND + 1];
-      } else if (B.kind == BC_CNS_ADIABATIC_NOSLIP) {  // :124-141
+      } else if (kind == BC_CNS_ADIABATIC_NOSLIP) {  // :124-141
 #pragma unroll
         for (int d = 0; d < ND; ++d) gp[d] = 0.0 - bp[d];
-      } else if (B.kind == BC_CNS_ADIABATIC_SLIP) {  // :164-190
+      } else if (kind == BC_CNS_ADIABATIC_SLIP) {  // :164-190
         const int ndir = gt.pos[i] >> 1;  // floor(boundary position w.r.t. the ghost / 2)
 #pragma unroll
         for (int d = 0; d < ND; ++d)
           if (d == ndir) gp[d] = 0.0 - bp[d];
-      } else if (B.kind == BC_CNS_ISOTHERMAL_NOSLIP || B.kind == BC_CPL_CNS_HEAT) {  // :209-228
+      } else if (kind == BC_CNS_ISOTHERMAL_NOSLIP || kind == BC_CPL_CNS_HEAT) {  // :209-228
         double Ts = B.v[0];
-        if (B.kind == BC_CPL_CNS_HEAT) {  // cns/coupling_conditions.hpp:28-42
+        if (kind == BC_CPL_CNS_HEAT) {  // cns/coupling_conditions.hpp:28-42
           if (gt.partner[i] < 0 || pv.q == nullptr) return;
           double ql[ND + 2];
 #pragma unroll
@@ -875,10 +893,15 @@ __global__ void __launch_bounds__(kBlock) k_stage(const double* __restrict__ qin
                                                   const double* __restrict__ sl, Geometry g, PhysConst pc,
                                                   const Scalars* __restrict__ sc, long long* dtmin) {
   constexpr int NV = nvars<ND, PHYS>();
-  chain_begin();
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int inst = tile_instance(g, blockIdx.x);
   const bool live = c < instance_end(g, inst);
+  int nb0[2 * ND];  // the cell's neighbours (heat)
+  if (PHYS == HEAT && live) {
+#pragma unroll
+    for (int p = 0; p < 2 * ND; ++p) nb0[p] = load_here(g.nbr + p * g.ld + c);
+  }
+  chain_begin();
   long long ord = kOrdMax;
   bool bad = false;
   if (live) {
@@ -964,7 +987,7 @@ __global__ void __launch_bounds__(kBlock) k_stage(const double* __restrict__ qin
       const double idx = 1 / dx;
 #pragma unroll
       for (int d = 0; d < ND; ++d) {
-        const int m = g.nbr[(2 * d) * ld + c], p = g.nbr[(2 * d + 1) * ld + c];
+        const int m = nb0[2 * d], p = nb0[2 * d + 1];
         double fm, fp;
         if (!HANG || m >= 0) {
           fm = idx * (__ldg(qin + m) - qc[0]);

@@ -45,20 +45,25 @@ template <int ND>
 __global__ void __launch_bounds__(kBlock) k_ghost_slopes(const double* __restrict__ q, Geometry g, GhostTables gt,
                                                          double* __restrict__ gsl, long long ngl) {
   constexpr int NV = ND + 2;
-  chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= gt.ng) return;
   const long long ld = g.ld;
-  const BcParam& B = gt.bcs[gt.bc_own[i]];
-  const long long b = B.kind == BC_PERIODIC ? gt.partner[i] : gt.bndry[i];
+  int b = -1, dg = 0, wall = 0, nb[2 * ND];
+  if (i < gt.ng) {
+    const BcParam& B = gt.bcs[load_here(gt.bc_own + i)];
+    wall = load_here(&B.wall);
+    dg = load_here(gt.pos + i) >> 1;
+    b = load_here(&B.kind) == BC_PERIODIC ? load_here(gt.partner + i) : load_here(gt.bndry + i);
+    if (b >= 0) {
+#pragma unroll
+      for (int p = 0; p < 2 * ND; ++p) nb[p] = load_here(g.nbr + p * ld + b);
+    }
+  }
+  chain_begin();
   if (b < 0) return;
-  const int dg = gt.pos[i] >> 1;
-  const bool wall = B.wall != 0;
   const double h2 = 2. * g.len[g.lvl[b]];
 #pragma unroll
   for (int sd = 0; sd < ND; ++sd) {
-    const int m = g.nbr[(2 * sd) * ld + b];
-    const int p = g.nbr[(2 * sd + 1) * ld + b];
+    const int m = nb[2 * sd], p = nb[2 * sd + 1];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       double s = (__ldg(q + v * ld + p) - __ldg(q + v * ld + m)) / h2;
@@ -222,10 +227,7 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
     return land + (size_t)v * S + s;
   };
 
-  chain_begin();
-  const double k = sc->dt / h;  // single grids only
   long long tile = blockIdx.x;
-  if (tile >= g.ntiles) return;
   if (tid == 0) {
     mbar_init(bar, 1);
     fence_mbar_init();
@@ -234,13 +236,13 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
 
   // halo cells (layer 1 then layer 2) of tile t this thread copies
   auto fetch_ids = [&](long long t, int* hid, int& o0, int& nh1) -> int {
-    o0 = __ldg(hg.halo_off + t);
-    const int nh = __ldg(hg.halo_off + t + 1) - o0;
-    nh1 = __ldg(ch.h1end + t) - o0;
+    o0 = load_here(hg.halo_off + t);
+    const int nh = load_here(hg.halo_off + t + 1) - o0;
+    nh1 = load_here(ch.h1end + t) - o0;
 #pragma unroll
     for (int k = 0; k < KH; ++k) {
       const int hh = tid + k * TB;
-      hid[k] = hh < nh ? __ldg(hg.halo_ids + o0 + hh) : 0;
+      hid[k] = hh < nh ? load_here(hg.halo_ids + o0 + hh) : 0;
     }
     return nh;
   };
@@ -318,8 +320,11 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
   };
 
   int hid[KH];
-  int o0, nh1;
-  int nh = fetch_ids(tile, hid, o0, nh1);
+  int o0 = 0, nh1 = 0, nh = 0;
+  if (tile < g.ntiles) nh = fetch_ids(tile, hid, o0, nh1);
+  chain_begin();
+  const double k = sc->dt / h;  // single grids only
+  if (tile >= g.ntiles) return;
   issue(tile, 0, hid, nh);
 
   for (int it = 0; tile < g.ntiles; tile += gridDim.x, ++it) {

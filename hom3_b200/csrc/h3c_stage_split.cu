@@ -91,13 +91,6 @@ __device__ __forceinline__ double* at32(double* row, unsigned c) {
   return reinterpret_cast<double*>(reinterpret_cast<char*>(row) + c * 8u);
 }
 
-// a load the compiler may not move ahead of the phase before it (its registers are needed there)
-__device__ __forceinline__ uint4 load_here(const uint4* p) {
-  uint4 r;
-  asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
-  return r;
-}
-
 }  // namespace
 
 template <int ND, class R, int MODE, bool HANG, bool FUSE>

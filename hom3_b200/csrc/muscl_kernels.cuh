@@ -38,14 +38,14 @@ __device__ __forceinline__ void prim_w(const double* __restrict__ q, long long l
   w[ND + 1] = gm1 * (__ldg(q + (ND + 1) * ld + c) - 0.5 * rho * um2);
 }
 
-// the face neighbours of interior cell c: f(n, d, side), side -1 (minus) / +1 (plus)
+// the face neighbours (entries nb of the table) of an interior cell: f(n, d, side), side -1 (minus) / +1 (plus)
 template <int ND, bool HANG, class F>
-__device__ __forceinline__ void for_each_face(const Geometry& g, long long c, F&& f) {
+__device__ __forceinline__ void for_each_face(const Geometry& g, const int* nb, F&& f) {
 #pragma unroll
   for (int d = 0; d < ND; ++d) {
 #pragma unroll
     for (int sd = 0; sd < 2; ++sd) {
-      const int n = g.nbr[(2 * d + sd) * g.ld + c];
+      const int n = nb[2 * d + sd];
       const int side = sd == 0 ? -1 : 1;
       if (!HANG || n >= 0) {
         f(n, d, side);
@@ -56,6 +56,14 @@ __device__ __forceinline__ void for_each_face(const Geometry& g, long long c, F&
       }
     }
   }
+}
+
+template <int ND, bool HANG, class F>
+__device__ __forceinline__ void for_each_face(const Geometry& g, long long c, F&& f) {
+  int nb[2 * ND];
+#pragma unroll
+  for (int p = 0; p < 2 * ND; ++p) nb[p] = g.nbr[p * g.ld + c];
+  for_each_face<ND, HANG>(g, nb, static_cast<F&&>(f));
 }
 
 // face point of the face between L (minus side) and R along d
@@ -91,10 +99,15 @@ __global__ void __launch_bounds__(kBlock) k_muscl_grad(const double* __restrict_
                                                        double* __restrict__ grad) {
   constexpr int NV = ND + 2;
   constexpr int NL = NV / SPLIT;  // this thread's variables: sub * NL ...
-  chain_begin();
-  int sub;
+  int sub, nb[2 * ND];
   const long long c = split_cell<SPLIT>(sub);
-  if (c >= g.n_int || c >= instance_end(g, tile_instance(g, c / kBlock))) return;  // also skips padding between instances
+  const bool live = c < g.n_int && c < instance_end(g, tile_instance(g, c / kBlock));  // not padding between instances
+  if (live) {
+#pragma unroll
+    for (int p = 0; p < 2 * ND; ++p) nb[p] = load_here(g.nbr + p * g.ld + c);
+  }
+  chain_begin();
+  if (!live) return;
   auto own = [&](const double* w, int v) { return SPLIT == 1 || sub == 0 ? w[v] : w[v + NV - NL]; };
   const long long ld = g.ld;
   const double gm1 = pc.gm1;
@@ -119,7 +132,7 @@ __global__ void __launch_bounds__(kBlock) k_muscl_grad(const double* __restrict_
 #pragma unroll
     for (int i = 0; i < ND; ++i) b[v][i] = 0.0;
   }
-  for_each_face<ND, HANG>(g, c, [&](int n, int, int) {
+  for_each_face<ND, HANG>(g, nb, [&](int n, int, int) {
     double wn[NV];
     prim_w<ND>(q, ld, n, gm1, wn);
     double dx[ND];
@@ -184,7 +197,7 @@ __global__ void __launch_bounds__(kBlock) k_muscl_grad(const double* __restrict_
     wmin[v] = wmin[v] - wc[v];
   }
   // one pass over the faces for all variables: the face offset is loaded once
-  for_each_face<ND, HANG>(g, c, [&](int n, int d, int side) {
+  for_each_face<ND, HANG>(g, nb, [&](int n, int d, int side) {
     double xf[ND];
     if (side < 0) face_point<ND>(g, xc, n, (int)c, d, xf);
     else face_point<ND>(g, xc, (int)c, n, d, xf);
@@ -253,12 +266,16 @@ __global__ void __launch_bounds__(kBlock) k_stage_muscl(const double* __restrict
   constexpr int NV = ND + 2;
   static_assert(SPLIT == 1 || SPLIT == ND, "a thread per cell, or per cell and direction");
   __shared__ double sacc[SPLIT > 1 ? NV : 1][SPLIT > 1 ? kBlock / SPLIT : 1];
-  chain_begin();
-  int sub;
+  int sub, nb[2 * ND];
   const long long c = split_cell<SPLIT>(sub);
   const int inst = c < g.n_int ? tile_instance(g, c / kBlock) : 0;
   bool live = c < g.n_int && c < instance_end(g, inst);
   const long long ld = g.ld;
+  if (live) {
+#pragma unroll
+    for (int p = 0; p < 2 * ND; ++p) nb[p] = load_here(g.nbr + p * ld + c);
+  }
+  chain_begin();
   double acc[NV];
 #pragma unroll
   for (int v = 0; v < NV; ++v) acc[v] = 0.0;
@@ -335,8 +352,8 @@ __global__ void __launch_bounds__(kBlock) k_stage_muscl(const double* __restrict
     for (int d = 0; d < ND; ++d) {
       if (SPLIT > 1 && d != sub) continue;  // the same for a whole warp
       double fm[NV], fp[NV];
-      side_flux(g.nbr[(2 * d) * ld + c], d, -1, fm);
-      side_flux(g.nbr[(2 * d + 1) * ld + c], d, 1, fp);
+      side_flux(nb[2 * d], d, -1, fm);
+      side_flux(nb[2 * d + 1], d, 1, fp);
 #pragma unroll
       for (int v = 0; v < NV; ++v) acc[v] = acc[v] + (fm[v] - fp[v]);
     }
