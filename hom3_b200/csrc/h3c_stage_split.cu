@@ -35,6 +35,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 
 #define H3C_DEVICE_FUNCTIONS_ONLY
 #include "fv_kernels.cuh"
@@ -501,9 +502,19 @@ void slaunch_m(int mode, bool hang, bool fuse, const SplitLaunch& a) {
 
 }  // namespace
 
+// The opt-in is the same for every grid and lasts as long as the device's
+// context, so a device's later grids skip its 32 calls (about 2 ms).
 bool split_prepare(int nd, bool mixed, size_t smem) {
-  if (nd == 2) return mixed ? sprep<2, float>(smem) : sprep<2, double>(smem);
-  return mixed ? sprep<3, float>(smem) : sprep<3, double>(smem);
+  constexpr int kDevices = 64;
+  static std::atomic<bool> done[kDevices][2][2];
+  int dev = 0;
+  const bool known = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kDevices;
+  std::atomic<bool>* d = known ? &done[dev][nd == 3][mixed] : nullptr;
+  if (d && d->load()) return true;
+  const bool ok = nd == 2 ? (mixed ? sprep<2, float>(smem) : sprep<2, double>(smem))
+                          : (mixed ? sprep<3, float>(smem) : sprep<3, double>(smem));
+  if (ok && d) d->store(true);
+  return ok;
 }
 
 void split_stage(int nd, bool mixed, int mode, bool hang, bool fuse, const double* qin, double* out,
