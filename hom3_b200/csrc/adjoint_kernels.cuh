@@ -379,8 +379,8 @@ template <int ND> __device__ __forceinline__ void side_from_shared(SideAD<ND>& S
 // ghost's condition Jacobian dq_ghost / dq_c = jac I (0 for interior cells).
 // skdt: alpha dt / length of each level.
 template <int ND>
-__device__ __forceinline__ void adj_neighbour(int nb, double kn_face, const double* __restrict__ q,
-                                              const double* __restrict__ lam, const double* skdt,
+__device__ __forceinline__ void adj_neighbour(int nb, double kn_face, const double* q,
+                                              const double* lam, const double* skdt,
                                               const Geometry& g, const GhostTables& gt, const PhysConst& pc,
                                               SideAD<ND>& Sn, double* kln, double& jac) {
   constexpr int NV = ND + 2;
@@ -405,8 +405,8 @@ __device__ __forceinline__ void adj_neighbour(int nb, double kn_face, const doub
   }
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
-    Sn.q[v] = __ldg(q + v * ld + nb);
-    kln[v] = own >= 0 ? kn * __ldg(lam + v * ld + own) : 0.0;
+    Sn.q[v] = q[v * ld + nb];
+    kln[v] = own >= 0 ? kn * lam[v * ld + own] : 0.0;
   }
   side_forward<ND>(Sn, pc.gamma, pc.gm1);
 }
@@ -417,10 +417,10 @@ __device__ __forceinline__ void adj_neighbour(int nb, double kn_face, const doub
 // gout_c = beta lam_c + [VJP of (q -> alpha k R(q)) with cotangent lam]_c + gamma_e extra_c + gamma_e2 extra2_c
 template <int ND, bool HANG>
 __global__ void __launch_bounds__(kBlock, H3C_ADJT_MINB)
-    k_adj_ausm(const double* __restrict__ q, const double* __restrict__ lam, double* __restrict__ gout,
-               const double* __restrict__ extra, const double* __restrict__ extra2, double alpha, double beta,
+    k_adj_ausm(const double* q, const double* lam, double* __restrict__ gout,
+               const double* extra, const double* extra2, double alpha, double beta,
                double gamma_e, double gamma_e2, Geometry g, GhostTables gt, PhysConst pc,
-               const double* __restrict__ dt) {
+               const double* dt) {
   constexpr int NV = ND + 2;
   constexpr int NS = 1 << (ND - 1);
   constexpr double W = ND == 2 ? 0.5 : 0.25;
@@ -452,14 +452,14 @@ __global__ void __launch_bounds__(kBlock, H3C_ADJT_MINB)
   SideAD<ND> Sc;
   if (live) {
 #pragma unroll
-    for (int v = 0; v < NV; ++v) Sc.q[v] = __ldg(q + v * ld + c);
+    for (int v = 0; v < NV; ++v) Sc.q[v] = q[v * ld + c];
     lc = g.lvl[c];
     const double kc = skdt[lc];
     side_forward<ND>(Sc, pc.gamma, pc.gm1);
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       ss[v * kBlock + tid] = Sc.q[v];
-      skl[v * kBlock + tid] = kc * __ldg(lam + v * ld + c);
+      skl[v * kBlock + tid] = kc * lam[v * ld + c];
     }
     ss[NV * kBlock + tid] = Sc.rinv;
     ss[(NV + 1) * kBlock + tid] = Sc.p;
@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(kBlock, H3C_ADJT_MINB)
   if (live) {
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-      double o = beta * __ldg(lam + v * ld + c) + acc[v];
+      double o = beta * lam[v * ld + c] + acc[v];
 #pragma unroll
       for (int d = 0; d < ND; ++d) o += sg[(d * NV + v) * kBlock + tid];
       if (extra) o += gamma_e * extra[v * ld + c];

@@ -213,6 +213,12 @@ __device__ __forceinline__ void flag_timeout(const Scalars* sc, int* status) {
 // The set-up tables do not change while kernels run, so what a block needs of
 // them first (a cell's neighbours, a ghost's boundary cell) is loaded before
 // the wait, by load_here: a load the compiler keeps where it stands.
+// Everything else a chained kernel reads -- states, scalars, slopes, gradients,
+// cotangents, recorded time steps -- may still be written by the kernel before
+// while it is already running, so it must not be read through the read-only
+// path (__ldg, const __restrict__), which asks for data that do not change as
+// long as the kernel lives and whose loads may move above the wait.  Plain
+// loads after chain_begin() are ordered by its memory clobber.
 __device__ __forceinline__ int load_here(const int* p) {
   int r;
   asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(r) : "l"(p) : "memory");
@@ -303,10 +309,10 @@ __device__ __forceinline__ void make_prim(Prim<R, ND>& P, R gamma, R gm1) {
 }
 
 template <class R, int ND>
-__device__ __forceinline__ void load_prim(Prim<R, ND>& P, const double* __restrict__ q, long long ld,
+__device__ __forceinline__ void load_prim(Prim<R, ND>& P, const double* q, long long ld,
                                           int c, R gamma, R gm1) {
 #pragma unroll
-  for (int v = 0; v < ND + 2; ++v) P.q[v] = (R)__ldg(q + v * ld + c);
+  for (int v = 0; v < ND + 2; ++v) P.q[v] = (R)q[v * ld + c];
   make_prim<R, ND>(P, gamma, gm1);
 }
 
@@ -486,8 +492,8 @@ __device__ __forceinline__ double cell_dt(const double* q, double h, const PhysC
 // cells on its way (1.45 M cells: one pass of 18 us for staging copies, a
 // gather and a CFL pass of 60).
 template <int ND, int PHYS, bool LOAD>
-__global__ void __launch_bounds__(kBlock) k_cfl(double* __restrict__ q, Geometry g, PhysConst pc, long long* dst,
-                                                const Scalars* sc, const double* __restrict__ src, long long src_ld,
+__global__ void __launch_bounds__(kBlock) k_cfl(double* q, Geometry g, PhysConst pc, long long* dst,
+                                                const Scalars* sc, const double* src, long long src_ld,
                                                 const int* __restrict__ idx) {
   constexpr int NV = nvars<ND, PHYS>();
   chain_begin();
@@ -499,7 +505,7 @@ __global__ void __launch_bounds__(kBlock) k_cfl(double* __restrict__ q, Geometry
     const int s = c >= g.n_tot ? -1 : idx ? __ldg(idx + c) : (int)c;
     if (s >= 0) {
 #pragma unroll
-      for (int v = 0; v < NV; ++v) qc[v] = __ldg(src + v * src_ld + s);
+      for (int v = 0; v < NV; ++v) qc[v] = src[v * src_ld + s];
 #pragma unroll
       for (int v = 0; v < NV; ++v) q[v * g.ld + c] = qc[v];
     }
@@ -665,7 +671,7 @@ __device__ __forceinline__ double partner_T(const BcParam& B, const PartnerView&
 // q: the state the condition is applied to (lhs or rhs); qlhs: the solver's
 // lhs, which the coupling conditions read temperatures from in both cases.
 template <int ND, int PHYS>
-__global__ void __launch_bounds__(kBlock) k_bc(double* __restrict__ q, const double* __restrict__ qlhs,
+__global__ void __launch_bounds__(kBlock) k_bc(double* q, const double* qlhs,
                                                Geometry g, GhostTables gt, PhysConst pc,
                                                const Scalars* sc, PartnerView pv, StepBegin begin) {
   constexpr int NV = nvars<ND, PHYS>();
@@ -835,7 +841,7 @@ __global__ void __launch_bounds__(kBlock) k_bc(double* __restrict__ q, const dou
 // (boundary_condition.hpp:63-67, cns/boundary_conditions.hpp:143-147,230-234).
 // ---------------------------------------------------------------------------
 template <int ND>
-__global__ void __launch_bounds__(kBlock) k_slopes(const double* __restrict__ q, Geometry g, GhostTables gt,
+__global__ void __launch_bounds__(kBlock) k_slopes(const double* q, Geometry g, GhostTables gt,
                                                    double* __restrict__ sl) {
   constexpr int NV = ND + 2;
   chain_begin();
@@ -860,7 +866,7 @@ __global__ void __launch_bounds__(kBlock) k_slopes(const double* __restrict__ q,
     const int p = g.nbr[(2 * sd + 1) * ld + b];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-      double s = (__ldg(q + v * ld + p) - __ldg(q + v * ld + m)) / h2;
+      double s = (q[v * ld + p] - q[v * ld + m]) / h2;
       if (wall && v < ND && sd != dg) s = -s;
       sl[(sd * NV + v) * ld + c] = s;
     }
@@ -889,9 +895,9 @@ template <int MODE> __device__ __forceinline__ double rk_combine(double q0, doub
 // HANG: the grid has coarse/fine faces (EXTENSION, not in hom3).
 // ---------------------------------------------------------------------------
 template <int ND, int PHYS, int FLUX, class R, int MODE, bool HANG, bool FUSE>
-__global__ void __launch_bounds__(kBlock) k_stage(const double* __restrict__ qin, double* out,
-                                                  const double* __restrict__ sl, Geometry g, PhysConst pc,
-                                                  const Scalars* __restrict__ sc, long long* dtmin) {
+__global__ void __launch_bounds__(kBlock) k_stage(const double* qin, double* out,
+                                                  const double* sl, Geometry g, PhysConst pc,
+                                                  const Scalars* sc, long long* dtmin) {
   constexpr int NV = nvars<ND, PHYS>();
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int inst = tile_instance(g, blockIdx.x);
@@ -910,7 +916,7 @@ __global__ void __launch_bounds__(kBlock) k_stage(const double* __restrict__ qin
     const double dx = g.len[g.lvl[c]];
     double qc[NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) qc[v] = __ldg(qin + v * ld + c);
+    for (int v = 0; v < NV; ++v) qc[v] = qin[v * ld + c];
     double acc[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) acc[v] = 0.0;
@@ -940,9 +946,9 @@ __global__ void __launch_bounds__(kBlock) k_stage(const double* __restrict__ qin
         }
 #pragma unroll
         for (int d = 0; d < ND; ++d) {
-          qm[d] = __ldg(qin + nm[d]);
+          qm[d] = qin[nm[d]];
           um[d] = __ldg(g.vel + d * ld + nm[d]);
-          qp[d] = __ldg(qin + np_[d]);
+          qp[d] = qin[np_[d]];
           up[d] = __ldg(g.vel + d * ld + np_[d]);
         }
 #pragma unroll
@@ -955,27 +961,27 @@ __global__ void __launch_bounds__(kBlock) k_stage(const double* __restrict__ qin
         const int m = g.nbr[(2 * d) * ld + c], p = g.nbr[(2 * d + 1) * ld + c];
         double fm, fp;
         if (!HANG || m >= 0) {
-          fm = adv_flux(__ldg(qin + m), qc[0], __ldg(g.vel + d * ld + m), uc);
+          fm = adv_flux(qin[m], qc[0], __ldg(g.vel + d * ld + m), uc);
         } else {
           const long long k = -m - 2;
           double ws = 0;
 #pragma unroll
           for (int j = 0; j < (1 << (ND - 1)); ++j) {
             const int n = g.sub[j * g.nsub + k];
-            const double f = adv_flux(__ldg(qin + n), qc[0], __ldg(g.vel + d * ld + n), uc);
+            const double f = adv_flux(qin[n], qc[0], __ldg(g.vel + d * ld + n), uc);
             ws = j == 0 ? f : ws + f;
           }
           fm = (ND == 2 ? 0.5 : 0.25) * ws;
         }
         if (!HANG || p >= 0) {
-          fp = adv_flux(qc[0], __ldg(qin + p), uc, __ldg(g.vel + d * ld + p));
+          fp = adv_flux(qc[0], qin[p], uc, __ldg(g.vel + d * ld + p));
         } else {
           const long long k = -p - 2;
           double ws = 0;
 #pragma unroll
           for (int j = 0; j < (1 << (ND - 1)); ++j) {
             const int n = g.sub[j * g.nsub + k];
-            const double f = adv_flux(qc[0], __ldg(qin + n), uc, __ldg(g.vel + d * ld + n));
+            const double f = adv_flux(qc[0], qin[n], uc, __ldg(g.vel + d * ld + n));
             ws = j == 0 ? f : ws + f;
           }
           fp = (ND == 2 ? 0.5 : 0.25) * ws;
@@ -990,25 +996,25 @@ __global__ void __launch_bounds__(kBlock) k_stage(const double* __restrict__ qin
         const int m = nb0[2 * d], p = nb0[2 * d + 1];
         double fm, fp;
         if (!HANG || m >= 0) {
-          fm = idx * (__ldg(qin + m) - qc[0]);
+          fm = idx * (qin[m] - qc[0]);
         } else {
           const long long k = -m - 2;
           double ws = 0;
 #pragma unroll
           for (int j = 0; j < (1 << (ND - 1)); ++j) {
-            const double f = idx * (__ldg(qin + g.sub[j * g.nsub + k]) - qc[0]);
+            const double f = idx * (qin[g.sub[j * g.nsub + k]] - qc[0]);
             ws = j == 0 ? f : ws + f;
           }
           fm = (ND == 2 ? 0.5 : 0.25) * ws;
         }
         if (!HANG || p >= 0) {
-          fp = idx * (qc[0] - __ldg(qin + p));
+          fp = idx * (qc[0] - qin[p]);
         } else {
           const long long k = -p - 2;
           double ws = 0;
 #pragma unroll
           for (int j = 0; j < (1 << (ND - 1)); ++j) {
-            const double f = idx * (qc[0] - __ldg(qin + g.sub[j * g.nsub + k]));
+            const double f = idx * (qc[0] - qin[g.sub[j * g.nsub + k]]);
             ws = j == 0 ? f : ws + f;
           }
           fp = (ND == 2 ? 0.5 : 0.25) * ws;
@@ -1025,7 +1031,7 @@ __global__ void __launch_bounds__(kBlock) k_stage(const double* __restrict__ qin
       R slc[PHYS == CNS ? ND * (ND + 2) : 1];
       if (PHYS == CNS) {
 #pragma unroll
-        for (int k = 0; k < ND * (ND + 2); ++k) slc[k] = (R)__ldg(sl + k * ld + c);
+        for (int k = 0; k < ND * (ND + 2); ++k) slc[k] = (R)sl[k * ld + c];
       }
       // flux of the face (l = a, r = b) with a or b the centre cell
       auto face = [&](const Prim<R, ND>& L, const Prim<R, ND>& Rt, const R* sL, const R* sR, R len_r, int d,
@@ -1043,7 +1049,7 @@ __global__ void __launch_bounds__(kBlock) k_stage(const double* __restrict__ qin
         load_prim<R, ND>(P, qin, ld, n, gamma, gm1);
         if (PHYS == CNS) {
 #pragma unroll
-          for (int k = 0; k < ND * (ND + 2); ++k) sn[k] = (R)__ldg(sl + k * ld + n);
+          for (int k = 0; k < ND * (ND + 2); ++k) sn[k] = (R)sl[k * ld + n];
         }
       };
 #pragma unroll
@@ -1144,8 +1150,8 @@ __global__ void __launch_bounds__(kBlock) k_stage(const double* __restrict__ qin
 // lost 8% in heat; left out.
 // ---------------------------------------------------------------------------
 template <int ND, int PHYS, int FLUX, int MODE, bool FUSE>
-__global__ void __launch_bounds__(kBlock) k_stage_scalar(const double* __restrict__ qin, double* out, Geometry g,
-                                                         PhysConst pc, const Scalars* __restrict__ sc,
+__global__ void __launch_bounds__(kBlock) k_stage_scalar(const double* qin, double* out, Geometry g,
+                                                         PhysConst pc, const Scalars* sc,
                                                          long long* dtmin) {
   static_assert(PHYS == HEAT || PHYS == ADVECTION, "one variable");
   constexpr bool ADV = PHYS == ADVECTION;
@@ -1164,7 +1170,7 @@ __global__ void __launch_bounds__(kBlock) k_stage_scalar(const double* __restric
   if (live) {
 #pragma unroll
     for (int p = 0; p < 2 * ND; ++p) nb[p] = __ldg(reinterpret_cast<const int2*>(g.nbr + p * ld + c));
-    q = __ldg(reinterpret_cast<const double2*>(qin + c));
+    q = *reinterpret_cast<const double2*>(qin + c);
     lv = __ldg(reinterpret_cast<const uchar2*>(g.lvl + c));
     if (ADV) {
 #pragma unroll
@@ -1184,7 +1190,7 @@ __global__ void __launch_bounds__(kBlock) k_stage_scalar(const double* __restric
       for (int j = 0; j < 2; ++j) {
         const int n = j ? nb[p].y : nb[p].x;
         const bool pair = both && (j ? n == (int)c : n == (int)c + 1);
-        qn[p][j] = pair ? (j ? q.x : q.y) : __ldg(qin + n);
+        qn[p][j] = pair ? (j ? q.x : q.y) : qin[n];
         if (ADV) un[p][j] = pair ? (j ? u[p >> 1].x : u[p >> 1].y) : __ldg(g.vel + (p >> 1) * ld + n);
       }
     }
@@ -1272,7 +1278,7 @@ __host__ __device__ constexpr size_t tile_smem_bytes() {
 
 template <int ND, int FLUX, class R, int MODE, bool HANG, bool FUSE>
 __global__ void __launch_bounds__(kBlock, 3) k_stage_tile(const double* __restrict__ qin, double* out, Geometry g,
-                                                       PhysConst pc, const Scalars* __restrict__ sc,
+                                                       PhysConst pc, const Scalars* sc,
                                                        long long* dtmin) {
   constexpr int NV = ND + 2;
   constexpr int NP = 3 * ND + 4;  // rows: q[ND+2], u[ND], p, a, M[ND]
@@ -1485,7 +1491,7 @@ __device__ __forceinline__ void face_state_global(FaceState<R, ND>& F, const dou
 template <int ND, class R, int MODE, bool HANG, bool FUSE, int TB = kBlock>
 __global__ void __launch_bounds__(TB, H3C_AUSM_MINB * kBlock / TB) k_stage_ausm(const double* __restrict__ qin,
                                                                               double* out, Geometry g, PhysConst pc,
-                                                                              const Scalars* __restrict__ sc,
+                                                                              const Scalars* sc,
                                                                               long long* dtmin) {
   constexpr int NV = ND + 2;
   constexpr int NS = 1 << (ND - 1);
@@ -1674,7 +1680,7 @@ __global__ void __launch_bounds__(TB, H3C_AUSM_MINB * kBlock / TB) k_stage_ausm(
 template <int ND, class R, int MODE, bool HANG, bool FUSE>
 __global__ void __launch_bounds__(kBlock, H3C_CELL_MINB) k_stage_ausm_cell(const double* __restrict__ qin, double* out,
                                                                           Geometry g, PhysConst pc,
-                                                                          const Scalars* __restrict__ sc,
+                                                                          const Scalars* sc,
                                                                           long long* dtmin) {
   constexpr int NV = ND + 2, NS = 1 << (ND - 1);
   constexpr double W = ND == 2 ? 0.5 : 0.25;

@@ -42,7 +42,7 @@ namespace h3c {
 // walls' sign flip of tangential velocity slopes: boundary_condition.hpp:63-67,
 // cns/boundary_conditions.hpp:143-147, 230-234), same arithmetic.
 template <int ND>
-__global__ void __launch_bounds__(kBlock) k_ghost_slopes(const double* __restrict__ q, Geometry g, GhostTables gt,
+__global__ void __launch_bounds__(kBlock) k_ghost_slopes(const double* q, Geometry g, GhostTables gt,
                                                          double* __restrict__ gsl, long long ngl) {
   constexpr int NV = ND + 2;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kBlock) k_ghost_slopes(const double* __restric
     const int m = nb[2 * sd], p = nb[2 * sd + 1];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-      double s = (__ldg(q + v * ld + p) - __ldg(q + v * ld + m)) / h2;
+      double s = (q[v * ld + p] - q[v * ld + m]) / h2;
       if (wall && v < ND && sd != dg) s = -s;
       gsl[(sd * NV + v) * ngl + i] = s;
     }
@@ -193,8 +193,8 @@ __device__ __forceinline__ long long cns_warp_dt(const double* q, bool live, dou
 // and directions: 12 of a tile's 36 warp-wide evaluations, against 4 of 28.
 template <int ND, class R, int MODE, bool FUSE, bool BRICK>
 __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
-    k_stage_cns_halo(const double* __restrict__ qin, double* out, Geometry g, CnsHaloGeom ch, PhysConst pc,
-                     const Scalars* __restrict__ sc, long long* dtmin, int* status) {
+    k_stage_cns_halo(const double* qin, double* out, Geometry g, CnsHaloGeom ch, PhysConst pc,
+                     const Scalars* sc, long long* dtmin, int* status) {
   constexpr int NV = ND + 2, NP = 2 * ND, TB = kHaloTile;
   constexpr int NPR = NV + ND + 2;  // q[nv], M[nd], p, a
   constexpr int SV = kCnsSlopeVars<ND>;
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
           for (int sd = 0; sd < ND; ++sd)
 #pragma unroll
             for (int v = 0; v < SV; ++v)
-              sl[(sd * SV + v) * S1 + s] = (R)__ldg(ch.gsl + (sd * NV + v) * ch.ngl + (n - g.n_int));
+              sl[(sd * SV + v) * S1 + s] = (R)ch.gsl[(sd * NV + v) * ch.ngl + (n - g.n_int)];
         } else {
 #pragma unroll
           for (int sd = 0; sd < ND; ++sd) {
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
     if (live) {
       double qc[NV], qo[NV];  // FP32: the landing area already holds the next tile
 #pragma unroll
-      for (int v = 0; v < NV; ++v) qc[v] = LIP ? *qslot(v, tid) : __ldg(qin + v * ld + c);
+      for (int v = 0; v < NV; ++v) qc[v] = LIP ? *qslot(v, tid) : qin[v * ld + c];
       if (MODE != 0) {
 #pragma unroll
         for (int v = 0; v < NV; ++v) qo[v] = g.q0[v * ld + c];

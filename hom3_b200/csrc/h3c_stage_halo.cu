@@ -76,7 +76,7 @@ __device__ __forceinline__ void face_state_of(const double* q, R gamma, R gm1, R
 template <int ND, class R, int MODE, bool HANG, bool FUSE>
 __global__ void __launch_bounds__(kHaloTile, 3)
     k_stage_halo(const double* __restrict__ qin, double* out, Geometry g, HaloGeom hg, PhysConst pc,
-                 const Scalars* __restrict__ sc, long long* dtmin, int* status) {
+                 const Scalars* sc, long long* dtmin, int* status) {
   constexpr int NV = ND + 2, NP = 2 * ND, NS = 1 << (ND - 1), TB = kHaloTile;
   constexpr int KH = kHaloMaxSlots / kHaloTile;  // halo entries one thread copies, at most
   constexpr int NFT = 2 * ND + 3;                // tile face-state rows: th[nv], p, M[nd]

@@ -96,8 +96,8 @@ __device__ __forceinline__ double* at32(double* row, unsigned c) {
 
 template <int ND, class R, int MODE, bool HANG, bool FUSE>
 __global__ void __launch_bounds__(kHaloTile, split_minb<ND, R>())
-    k_stage_split(const double* __restrict__ qin, double* out, Geometry g, SplitGeom sg, PhysConst pc,
-                  const Scalars* __restrict__ sc, long long* dtmin) {
+    k_stage_split(const double* qin, double* out, Geometry g, SplitGeom sg, PhysConst pc,
+                  const Scalars* sc, long long* dtmin) {
   constexpr int NV = ND + 2, NP = 2 * ND, NS = 1 << (ND - 1), TB = kHaloTile;
   constexpr int HM = split_slots<ND, R>(), S = TB + HM;
   constexpr double W = ND == 2 ? 0.5 : 0.25;
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kHaloTile, split_minb<ND, R>())
   };
   auto fetch = [&](unsigned n, double* q) {
 #pragma unroll
-    for (int v = 0; v < NV; ++v) q[v] = __ldg(at32(qin + v * ld, n));
+    for (int v = 0; v < NV; ++v) q[v] = *at32(qin + v * ld, n);
   };
 
   for (long long tile = blockIdx.x; tile < g.ntiles; tile += gridDim.x) {
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(kHaloTile, split_minb<ND, R>())
       double o[NV];
 #pragma unroll
       for (int v = 0; v < NV; ++v)
-        o[v] = rk_combine<MODE>(MODE == 0 ? 0.0 : qo[v], __ldg(at32(qin + v * ld, c)), k * acc[v]);
+        o[v] = rk_combine<MODE>(MODE == 0 ? 0.0 : qo[v], *at32(qin + v * ld, c), k * acc[v]);
 #pragma unroll
       for (int v = 0; v < NV; ++v) *at32(out + v * ld, c) = o[v];
       if (FUSE) {

@@ -89,7 +89,7 @@ __device__ __forceinline__ void face_state_of(const double* qn, int d, R gamma, 
 template <int ND, class R, int MODE, bool HANG, bool FUSE>
 __global__ void __launch_bounds__(kBlock, H3C_WARP_MINB)
     k_stage_ausm_warp(const double* __restrict__ qin, double* out, Geometry g, PhysConst pc,
-                      const Scalars* __restrict__ sc, long long* dtmin) {
+                      const Scalars* sc, long long* dtmin) {
   constexpr int NV = ND + 2, NS = 1 << (ND - 1);
   constexpr double W = ND == 2 ? 0.5 : 0.25;
   extern __shared__ __align__(16) unsigned char warp_smem_raw[];

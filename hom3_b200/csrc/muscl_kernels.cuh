@@ -24,18 +24,18 @@
 namespace h3c {
 
 template <int ND>
-__device__ __forceinline__ void prim_w(const double* __restrict__ q, long long ld, long long c, double gm1,
+__device__ __forceinline__ void prim_w(const double* q, long long ld, long long c, double gm1,
                                        double* w) {
-  const double rho = __ldg(q + ND * ld + c);
+  const double rho = q[ND * ld + c];
   const double rinv = nr_rcp(rho);
   double um2 = 0.0;
 #pragma unroll
   for (int d = 0; d < ND; ++d) {
-    w[d] = __ldg(q + d * ld + c) * rinv;
+    w[d] = q[d * ld + c] * rinv;
     um2 = d == 0 ? w[d] * w[d] : um2 + w[d] * w[d];
   }
   w[ND] = rho;
-  w[ND + 1] = gm1 * (__ldg(q + (ND + 1) * ld + c) - 0.5 * rho * um2);
+  w[ND + 1] = gm1 * (q[(ND + 1) * ld + c] - 0.5 * rho * um2);
 }
 
 // the face neighbours (entries nb of the table) of an interior cell: f(n, d, side), side -1 (minus) / +1 (plus)
@@ -94,7 +94,7 @@ template <int SPLIT> __device__ __forceinline__ long long split_cell(int& sub) {
 // instructions: 256^2 cells are 3.5 warps per scheduler, of which the FP64
 // pipe sees a third.
 template <int ND, bool HANG, int SPLIT>
-__global__ void __launch_bounds__(kBlock) k_muscl_grad(const double* __restrict__ q, const double* __restrict__ xc,
+__global__ void __launch_bounds__(kBlock) k_muscl_grad(const double* q, const double* __restrict__ xc,
                                                        Geometry g, PhysConst pc, double limiter_k,
                                                        double* __restrict__ grad) {
   constexpr int NV = ND + 2;
@@ -258,10 +258,10 @@ __device__ __forceinline__ void prim_from_w(const double* w, R gamma, R igm1, Pr
 // SPLIT 2 (2D): the two directions of a cell by two threads; the second's sum
 // goes to the first through shared memory.
 template <int ND, class R, int MODE, bool HANG, bool FUSE, int SPLIT>
-__global__ void __launch_bounds__(kBlock) k_stage_muscl(const double* __restrict__ qin, double* out,
-                                                        const double* __restrict__ grad,
+__global__ void __launch_bounds__(kBlock) k_stage_muscl(const double* qin, double* out,
+                                                        const double* grad,
                                                         const double* __restrict__ xc, Geometry g, PhysConst pc,
-                                                        const Scalars* __restrict__ sc, long long* dtmin,
+                                                        const Scalars* sc, long long* dtmin,
                                                         const int* __restrict__ gsrc) {
   constexpr int NV = ND + 2;
   static_assert(SPLIT == 1 || SPLIT == ND, "a thread per cell, or per cell and direction");
@@ -289,10 +289,10 @@ __global__ void __launch_bounds__(kBlock) k_stage_muscl(const double* __restrict
     const R gamma = (R)pc.gamma, igm1 = R(1) / (R)pc.gm1;
     double wc[NV], Gc[NV * ND], xcc[ND];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) qc[v] = __ldg(qin + v * ld + c);
+    for (int v = 0; v < NV; ++v) qc[v] = qin[v * ld + c];
     prim_w<ND>(qin, ld, c, gm1, wc);
 #pragma unroll
-    for (int k = 0; k < NV * ND; ++k) Gc[k] = __ldg(grad + k * ld + c);
+    for (int k = 0; k < NV * ND; ++k) Gc[k] = grad[k * ld + c];
 #pragma unroll
     for (int k = 0; k < ND; ++k) xcc[k] = __ldg(xc + k * ld + c);
     // flux of the face between c and n along d (side: where n lies), into f
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(kBlock) k_stage_muscl(const double* __restrict
         wcf[v] = s;
         double t = wn[v];
 #pragma unroll
-        for (int k = 0; k < ND; ++k) t = t + __ldg(grad + (v * ND + k) * ld + gn) * (xf[k] - xn[k]);
+        for (int k = 0; k < ND; ++k) t = t + grad[(v * ND + k) * ld + gn] * (xf[k] - xn[k]);
         wnf[v] = t;
       }
       if (!(wcf[ND] > 0) || !(wcf[ND + 1] > 0) || !(wnf[ND] > 0) || !(wnf[ND + 1] > 0)) {

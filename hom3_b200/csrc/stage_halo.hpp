@@ -96,7 +96,7 @@ struct CnsHaloGeom {
   const int* __restrict__ h1end;             // [ntiles] end of tile t's layer 1 in halo_ids
   const unsigned short* __restrict__ hnb;    // [halo_ids entries][2nd] slots of a layer-1 cell's face
                                              // neighbours (0xffff: that slope is not needed)
-  const double* __restrict__ gsl;            // [nd * nv][ngl] slopes of the ghost cells
+  const double* gsl;                         // [nd * nv][ngl] slopes of the ghost cells (the kernel before writes them)
   long long ngl;                             // leading dimension of gsl
   int h1max;                                 // layer-1 slots reserved per tile (multiple of 32)
   // brick grids (else nullptr): per tile the minus faces on its border -- cell slot, neighbour slot << 8,
