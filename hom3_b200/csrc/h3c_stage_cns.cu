@@ -134,17 +134,21 @@ __device__ __forceinline__ void ausm_subsonic_first(const Prim<R, ND>& L, const 
     if (v == d) f[v] = f[v] + pi;
 }
 
-// cell_dt of CNS (fv_kernels.cuh) over a warp's cells.  On one level each of
-// its two parts falls as its argument grows, division by division, so the
-// least time step of a warp is that of its largest wave speed and largest
-// viscous coefficient, to the bit.  The coefficient's own three divisions and
-// square root are left out where the viscous part cannot be the smaller one
-// for any cell: an estimate by reciprocals (within a few ulp, against a margin
-// of 1e-9) of the warp's largest decides.  128^3 Taylor-Green, second RK2
-// stage: 347.6 us with both parts in every cell, 336.8 here.
+// cell_dt of CNS (fv_kernels.cuh) over a warp's cells: per lane a value whose
+// minimum over the warp is the cells' minimum, to the bit.  On one level the
+// convective part falls as the wave speed grows, division by division, so the
+// warp's least is that of its largest wave speed; and the viscous part, three
+// divisions and a square root more, is left out where it cannot be the
+// smaller one for any cell: an estimate by reciprocals (within a few ulp,
+// against a margin of 1e-9) of the warp's largest decides.  A cell that is no
+// physical state, or has no wave speed or estimate, sends its warp to cell_dt
+// in every cell (a NaN state's time step lies below zero, and a maximum drops
+// it).  128^3 Taylor-Green, second RK2 stage: 347.6 us with both parts in
+// every cell, 336.8 here.
 template <int ND>
 __device__ __forceinline__ long long cns_warp_dt(const double* q, bool live, double h, const PhysConst& pc, bool& bad) {
   Prim<double, ND> P;
+  const double kInf = __longlong_as_double(0x7ff0000000000000LL);
   double S = -1.7976931348623157e308, est = S;
   if (live) {
 #pragma unroll
@@ -159,30 +163,17 @@ __device__ __forceinline__ long long cns_warp_dt(const double* q, bool live, dou
     const double rinv = nr_rcp(P.q[ND]);
     const double T = pc.gamma * P.p * rinv;
     est = (T * (T * nr_rsqrt(T))) * pc.sOverTrefP1 * nr_rcp(T + pc.sOverTref) * rinv;
-    if (bad) est = 1e300;  // no estimate: the exact path
+    if (bad || !(S > 0.0) || !(est > 0.0)) est = kInf;  // cell_dt decides
   }
   for (int w = 16; w > 0; w >>= 1) {
     S = fmax(S, __shfl_xor_sync(0xffffffffu, S, w));
     est = fmax(est, __shfl_xor_sync(0xffffffffu, est, w));
   }
-  if (!(S > 0.0)) return kOrdMax;  // no live cell, or none with a wave speed
-  const double dt_inv = pc.cfl * h / S;
-  double dt = dt_inv;
   // dt_v = cflv h / (2 S_visc), S_visc = coeff max(1 / Re0, 1 / (Re0 Pr0 gm1)), coeff = est / h
   const double worst = est * fmax(1.0, nr_rcp(pc.Pr0 * pc.gm1)) * nr_rcp(pc.Re0 * h);
-  if (!(pc.cflv * S > (2.0 + 1e-9) * pc.cfl * worst)) {
-    double coeff = -1.7976931348623157e308;
-    if (live) {
-      const double T = pc.gamma * P.p / P.q[ND];
-      const double c = sutherland<double>(T, pc.sOverTref, pc.sOverTrefP1) / (P.q[ND] * h);
-      if (c > coeff) coeff = c;  // NaN never wins
-    }
-    for (int w = 16; w > 0; w >>= 1) coeff = fmax(coeff, __shfl_xor_sync(0xffffffffu, coeff, w));
-    const double a1 = coeff / pc.Re0, a2 = coeff / (pc.Re0 * pc.Pr0 * pc.gm1);
-    const double S_visc = (a1 < a2) ? a2 : a1;
-    const double dt_v = pc.cflv * h / (2 * S_visc);
-    dt = (dt_v < dt_inv) ? dt_v : dt_inv;
-  }
+  const bool convective = S > 0.0 && pc.cflv * S > (2.0 + 1e-9) * pc.cfl * worst;  // the same in every lane
+  if (!convective && !live) return kOrdMax;
+  const double dt = convective ? pc.cfl * h / S : cell_dt<ND, CNS>(q, h, pc);
   return isnan(dt) ? kOrdMax : dbl_to_ord(dt);
 }
 
