@@ -2425,6 +2425,11 @@ int h3c_adjoint(h3c_solver s, int64_t nsteps, int64_t every, const double* dJ_dq
   double* m_gbar = m_dl1 + Q;
   double* m_bbar = m_gbar + s->nd * Q;
   int* m_owner = reinterpret_cast<int*>(m_bbar + s->nd * Q);
+  // what can fail comes before the first step: the staging buffer, if one of the caller's arrays needs it
+  for (const double* cols : {dJ_dqN, (const double*)dJ_dq0}) {
+    if (in_place(s, cols, s->n_caller)) continue;
+    if (int rc = ensure_stage(s, s->n_caller)) return rc;
+  }
   const long long last0 = (nck - 1) * every;  // first step of the last segment
   // ---- forward: the solver's own step (CFL dt), checkpoints, dt record ----
   const bool fuse = !s->unfused_dt;
