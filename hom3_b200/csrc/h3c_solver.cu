@@ -107,7 +107,7 @@ struct h3c_solver_s {
   std::vector<long long> dev2caller, caller2dev;
   Scalars* d_sc = nullptr;
   Scalars* h_sc = nullptr;  // pinned host copy of instance 0's scalars (the per-step dt read-back)
-  HostScalars* h_mirror = nullptr;  // what the steps' kernels write of them (mapped pinned memory)
+  HostScalars* h_mirror = nullptr;  // what the steps' kernels write of them (behind h_sc in the same pinned block)
   bool mirror_valid = false;        // the last thing that changed the scalars was a step that wrote the mirror
   const double* stage_q0 = nullptr; // start state of the stage being launched (Geometry::q0)
   bool unfused_dt = false;  // a condition rewrites interior cells (vortex)
@@ -694,18 +694,16 @@ int h3c_create(const h3c_desc* d, h3c_solver* out) {
     g_last_error = std::string("h3c_create: cudaMalloc: ") + cudaGetErrorString(e);
     return H3C_E_NOMEM;
   }
-  // a direct DMA target for the step scalars (a pageable one is staged by the driver)
-  if (cudaMallocHost(&s->h_sc, sizeof(Scalars)) != cudaSuccess) {
+  // one pinned block: a direct DMA target for the step scalars (a pageable one is staged by the driver), and the
+  // scalars the steps' kernels write through its device address (the same one under unified addressing)
+  void* dev_block = nullptr;
+  if (cudaMallocHost(&s->h_sc, sizeof(Scalars) + sizeof(HostScalars)) != cudaSuccess) {
     cudaGetLastError();
     s->h_sc = nullptr;
-  }
-  // written by the steps' kernels through its device address (the same one under unified addressing)
-  void* mirror_dev = nullptr;
-  if (cudaHostAlloc((void**)&s->h_mirror, sizeof(HostScalars), cudaHostAllocMapped) != cudaSuccess ||
-      cudaHostGetDevicePointer(&mirror_dev, s->h_mirror, 0) != cudaSuccess || mirror_dev != (void*)s->h_mirror) {
+  } else if (cudaHostGetDevicePointer(&dev_block, s->h_sc, 0) == cudaSuccess && dev_block == (void*)s->h_sc) {
+    s->h_mirror = reinterpret_cast<HostScalars*>(s->h_sc + 1);
+  } else {
     cudaGetLastError();
-    if (s->h_mirror) cudaFreeHost(s->h_mirror);
-    s->h_mirror = nullptr;
   }
   k_init_time<<<1, 1, 0, s->stream>>>(s->d_sc, d->time_end, 1, s->h_mirror);
   *out = s.release();
@@ -718,7 +716,6 @@ int h3c_destroy(h3c_solver s) {
   free_grid(s);
   dfree(s->d_sc);
   if (s->h_sc) cudaFreeHost(s->h_sc);
-  if (s->h_mirror) cudaFreeHost(s->h_mirror);
   for (auto& r : s->prof_rec) { cudaEventDestroy(r.second.first); cudaEventDestroy(r.second.second); }
   for (auto e : s->ev_pool) cudaEventDestroy(e);
   if (s->stream && s->own_stream) cudaStreamDestroy(s->stream);
@@ -1083,7 +1080,7 @@ static int set_grids(h3c_solver s, int ninst, const h3c_grid* grids) {
     const size_t smem = halo_smem_bytes(nd, mixed, HH.hmax);
     const int bps = halo_prepare(nd, mixed, smem);
     const size_t ssmem = split_smem_bytes(nd, mixed);
-    const bool split = split_prepare(nd, mixed, ssmem);
+    const bool split = split_prepare(nd, mixed, stage_modes(s->desc.time_integration), nsub > 0, ssmem);
     if (bps > 0 || split) {
       H3C_CUDA(s, cudaMalloc(&s->d_lnb, sizeof(unsigned short) * HH.lnb.size()));
       H3C_CUDA(s, cudaMalloc(&s->d_hids, sizeof(int) * HH.ids.size()));
@@ -1118,7 +1115,7 @@ static int set_grids(h3c_solver s, int ninst, const h3c_grid* grids) {
     for (int brick = CH.brick ? 1 : 0; brick >= 0 && bps == 0; --brick) {
       CH.brick = brick != 0;
       smem = cns_halo_smem_bytes(nd, mixed, CH.base.hmax, CH.h1max, CH.brick);
-      bps = smem <= 227 * 1024 ? cns_halo_prepare(nd, mixed, smem, CH.brick) : 0;
+      bps = smem <= 227 * 1024 ? cns_halo_prepare(nd, mixed, stage_modes(s->desc.time_integration), smem, CH.brick) : 0;
     }
     if (bps > 0 && CH.brick) {
       H3C_CUDA(s, cudaMalloc(&s->d_blist, sizeof(unsigned) * CH.blist.size()));

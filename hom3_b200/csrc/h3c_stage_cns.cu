@@ -657,18 +657,24 @@ int cprep_one(size_t smem) {
   }
   return nb;
 }
+// the least over the variants the solver launches (a variant is loaded by its first call: 8 of them took a first
+// grid 20 ms)
 template <int ND, class R, int MODE, bool BRICK>
 int cprep_f(size_t smem) {
   return std::min(cprep_one<ND, R, MODE, false, BRICK>(smem), cprep_one<ND, R, MODE, true, BRICK>(smem));
 }
 template <int ND, class R, bool BRICK>
-int cprep_m(size_t smem) {
-  return std::min(std::min(cprep_f<ND, R, 0, BRICK>(smem), cprep_f<ND, R, 2, BRICK>(smem)),
-                  std::min(cprep_f<ND, R, 3, BRICK>(smem), cprep_f<ND, R, 4, BRICK>(smem)));
+int cprep_m(unsigned modes, size_t smem) {
+  int n = 1 << 30;
+  if (modes & 1u) n = std::min(n, cprep_f<ND, R, 0, BRICK>(smem));
+  if (modes & 4u) n = std::min(n, cprep_f<ND, R, 2, BRICK>(smem));
+  if (modes & 8u) n = std::min(n, cprep_f<ND, R, 3, BRICK>(smem));
+  if (modes & 16u) n = std::min(n, cprep_f<ND, R, 4, BRICK>(smem));
+  return n;
 }
 template <int ND, class R>
-int cprep(size_t smem, bool brick) {
-  return brick ? cprep_m<ND, R, true>(smem) : cprep_m<ND, R, false>(smem);
+int cprep(unsigned modes, size_t smem, bool brick) {
+  return brick ? cprep_m<ND, R, true>(modes, smem) : cprep_m<ND, R, false>(modes, smem);
 }
 
 struct CnsLaunch {
@@ -712,9 +718,9 @@ void claunch_m(int mode, bool fuse, const CnsLaunch& a) {
 
 }  // namespace
 
-int cns_halo_prepare(int nd, bool mixed, size_t smem, bool brick) {
-  if (nd == 2) return mixed ? cprep<2, float>(smem, brick) : cprep<2, double>(smem, brick);
-  return mixed ? cprep<3, float>(smem, brick) : cprep<3, double>(smem, brick);
+int cns_halo_prepare(int nd, bool mixed, unsigned modes, size_t smem, bool brick) {
+  if (nd == 2) return mixed ? cprep<2, float>(modes, smem, brick) : cprep<2, double>(modes, smem, brick);
+  return mixed ? cprep<3, float>(modes, smem, brick) : cprep<3, double>(modes, smem, brick);
 }
 
 void cns_halo_stage(int nd, bool mixed, int mode, bool fuse, const double* qin, double* out, const Geometry& g,

@@ -35,7 +35,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 
 #define H3C_DEVICE_FUNCTIONS_ONLY
 #include "fv_kernels.cuh"
@@ -459,13 +458,14 @@ bool sprep_one(size_t smem) {
   return true;
 }
 template <int ND, class R, int MODE>
-bool sprep_m(size_t smem) {
-  return sprep_one<ND, R, MODE, false, false>(smem) && sprep_one<ND, R, MODE, false, true>(smem) &&
-         sprep_one<ND, R, MODE, true, false>(smem) && sprep_one<ND, R, MODE, true, true>(smem);
+bool sprep_m(size_t smem, bool hang) {
+  return hang ? sprep_one<ND, R, MODE, true, false>(smem) && sprep_one<ND, R, MODE, true, true>(smem)
+              : sprep_one<ND, R, MODE, false, false>(smem) && sprep_one<ND, R, MODE, false, true>(smem);
 }
 template <int ND, class R>
-bool sprep(size_t smem) {
-  return sprep_m<ND, R, 0>(smem) && sprep_m<ND, R, 2>(smem) && sprep_m<ND, R, 3>(smem) && sprep_m<ND, R, 4>(smem);
+bool sprep(size_t smem, unsigned modes, bool hang) {
+  return (!(modes & 1u) || sprep_m<ND, R, 0>(smem, hang)) && (!(modes & 4u) || sprep_m<ND, R, 2>(smem, hang)) &&
+         (!(modes & 8u) || sprep_m<ND, R, 3>(smem, hang)) && (!(modes & 16u) || sprep_m<ND, R, 4>(smem, hang));
 }
 
 struct SplitLaunch {
@@ -502,19 +502,14 @@ void slaunch_m(int mode, bool hang, bool fuse, const SplitLaunch& a) {
 
 }  // namespace
 
-// The opt-in is the same for every grid and lasts as long as the device's
-// context, so a device's later grids skip its 32 calls (about 2 ms).
-bool split_prepare(int nd, bool mixed, size_t smem) {
-  constexpr int kDevices = 64;
-  static std::atomic<bool> done[kDevices][2][2];
-  int dev = 0;
-  const bool known = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kDevices;
-  std::atomic<bool>* d = known ? &done[dev][nd == 3][mixed] : nullptr;
-  if (d && d->load()) return true;
-  const bool ok = nd == 2 ? (mixed ? sprep<2, float>(smem) : sprep<2, double>(smem))
-                          : (mixed ? sprep<3, float>(smem) : sprep<3, double>(smem));
-  if (ok && d) d->store(true);
-  return ok;
+// 48 KB are a block's without an opt-in: only 3D FP64 (56 KB) needs one, for
+// the variants the solver launches (each is loaded by its first call, which
+// for all 16 of a dimension and precision took a first grid 2 ms).
+bool split_prepare(int nd, bool mixed, unsigned modes, bool hang, size_t smem) {
+  constexpr size_t kFree = 48 * 1024, kStatic = 1024;  // the kernel's static arrays are smaller
+  if (smem + kStatic <= kFree) return true;
+  if (nd == 2) return mixed ? sprep<2, float>(smem, modes, hang) : sprep<2, double>(smem, modes, hang);
+  return mixed ? sprep<3, float>(smem, modes, hang) : sprep<3, double>(smem, modes, hang);
 }
 
 void split_stage(int nd, bool mixed, int mode, bool hang, bool fuse, const double* qin, double* out,

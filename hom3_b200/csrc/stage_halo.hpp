@@ -25,6 +25,11 @@ namespace h3c {
 constexpr int kHaloTile = 256;              // cells per tile = threads per block
 constexpr int kHaloMaxSlots = 1024;         // halo entries a tile may hold in shared memory
 constexpr unsigned short kGroupBit = 0x8000;
+
+// The stage modes (rk_combine) of a time integration (h3c_time_integration), one bit each.
+constexpr unsigned stage_modes(int time_integration) {
+  return time_integration == 0 ? 1u : time_integration == 1 ? 1u | 1u << 2 : 1u | 1u << 3 | 1u << 4;
+}
 // Euler halo entries are (cell, direction, side) triples: the id word carries
 // the cell in its low 29 bits, the face direction it is read across in bits
 // 29-30 and in bit 31 whether it lies on the plus side of that face (the CNS
@@ -117,7 +122,7 @@ struct CnsHaloHost {
 bool halo_build_cns(int nd, long long ld, long long n_int, long long ntiles, const std::vector<long long>& tile_end,
                     const int* nbr, CnsHaloHost& H);
 size_t cns_halo_smem_bytes(int nd, bool mixed, int hmax, int h1max, bool brick);
-int cns_halo_prepare(int nd, bool mixed, size_t smem, bool brick);
+int cns_halo_prepare(int nd, bool mixed, unsigned modes, size_t smem, bool brick);
 // the ghost-slope pass and the stage; h = the grid's (single) cell length
 void cns_halo_stage(int nd, bool mixed, int mode, bool fuse, const double* qin, double* out, const Geometry& g,
                     const GhostTables& gt, const CnsHaloGeom& h, const PhysConst& pc, const Scalars* sc,

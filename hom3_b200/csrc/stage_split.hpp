@@ -20,9 +20,10 @@ void split_pack(int nd, const unsigned short* lnb, const unsigned char* lvl, lon
 
 // Dynamic shared memory of one block.
 size_t split_smem_bytes(int nd, bool mixed);
-// Opts every instantiation for nd / precision into its dynamic shared memory
-// (outside capture); false when the kernel cannot be launched.
-bool split_prepare(int nd, bool mixed, size_t smem);
+// Opts the instantiations a solver launches (stage_modes, with or without
+// coarse/fine faces) into their dynamic shared memory where that needs an
+// opt-in (outside capture); false when the kernel cannot be launched.
+bool split_prepare(int nd, bool mixed, unsigned modes, bool hang, size_t smem);
 
 // One stage: out = rk_combine<mode>(g.q0, qin, dt/dx R(qin)), with the fused
 // next-step CFL minimum into dtmin when fuse; grid blocks take the tiles round-robin.
