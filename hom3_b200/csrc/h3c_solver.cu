@@ -135,7 +135,7 @@ struct h3c_solver_s {
   bool split_ok = false;
   void* d_pack = nullptr;
   size_t split_smem = 0;
-  // CNS tile kernel (h3c_stage_cns.cu): its tables reuse d_lnb / d_hids / d_hoff
+  // CNS tile kernel (stage_cns.cuh): its tables reuse d_lnb / d_hids / d_hoff
   bool cns_ok = false;
   int* d_h1end = nullptr;
   unsigned *d_blist = nullptr, *d_bsel = nullptr;  // brick grids: border lists

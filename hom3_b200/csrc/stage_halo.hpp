@@ -88,7 +88,7 @@ void halo_stage(int nd, bool mixed, int mode, bool hang, bool fuse, const double
                 int* status, int grid, size_t smem, cudaStream_t st);
 
 // ---------------------------------------------------------------------------
-// CNS (AUSM + three-point viscous flux) on the same tiles (h3c_stage_cns.cu).
+// CNS (AUSM + three-point viscous flux) on the same tiles (stage_cns.cuh).
 // The viscous flux reads the transverse slopes of both face cells, so the
 // tables add, per tile, a second halo layer: the cells the slopes of the
 // first layer read (the tile's edge-diagonal neighbours, and ghosts next to
@@ -115,7 +115,7 @@ struct CnsHaloHost {
   std::vector<int> h1end;
   std::vector<unsigned short> hnb;
   int h1max = 0;
-  bool brick = false;                        // every tile fits the brick variant (h3c_stage_cns.cu)
+  bool brick = false;                        // every tile fits the brick variant (stage_cns.cuh)
   std::vector<unsigned> blist, bsel;
 };
 
