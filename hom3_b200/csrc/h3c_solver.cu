@@ -413,8 +413,45 @@ void launch_grad(h3c_solver s, const double* q, bool ghosts_too) {
   }
 }
 
+// Two cells per thread in the stages of heat and advection (k_stage_scalar): one grid without coarse/fine faces
+// (neighbour entries are cells then, never groups), from one full wave of k_stage's blocks on; below, a thread per
+// cell finishes sooner (32,768 heat cells: 7.0 us against 8.5).
+bool scalar_pairs(h3c_solver s) {
+  return (s->desc.physics == H3C_HEAT || s->desc.physics == H3C_ADVECTION) && s->nsub == 0 && s->n_inst == 1 &&
+         s->n_int >= 6LL * kBlock * num_sms();
+}
+
+// The stage kernels, by the codes h3c_kernel_info reports.
+enum StageKernel {
+  ST_PER_CELL = 0,  // k_stage, k_stage_scalar, k_stage_muscl
+  ST_SPLIT = 1,     // k_stage_split
+  ST_HALO = 2,      // k_stage_halo; CNS: k_stage_cns_halo
+  ST_CELL = 3,      // k_stage_ausm_cell
+  ST_WARP = 4,      // k_stage_ausm_warp
+  ST_LANE512 = 5,   // k_stage_ausm, 512-cell tiles
+  ST_LANE = 6,      // k_stage_ausm, 256-cell tiles
+  ST_TILE = 7,      // k_stage_tile (LLF)
+};
+bool cns_tile_active(const h3c_solver s) { return s->desc.physics == H3C_CNS && s->tile && s->halo && s->cns_ok; }
+
+// The per-lane kernel on 256-cell tiles reads no halo tables: it runs where they or the split kernel's shared
+// memory could not be had (2^29 cells and more), ahead of the per-cell kernel (tree, stage 1 / 2 in us: 98.8 /
+// 111.5 against 100.8 / 120.0), and for kernel 0 with the halo tables switched off.
+StageKernel stage_kernel(const h3c_solver s) {
+  if (cns_tile_active(s)) return ST_HALO;
+  if (s->desc.physics != H3C_EULER || s->desc.reconstruction == H3C_RECON_MUSCL || !s->tile) return ST_PER_CELL;
+  if (s->desc.flux != H3C_FLUX_AUSM) return ST_TILE;
+  const int k = s->euler_kernel;
+  if (k == 3 && s->warp_bps > 0) return ST_WARP;
+  if (k == 2 || k == 3) return ST_CELL;
+  if (k == 0 && s->halo && s->halo_ok) return ST_HALO;
+  if (k == 4 && s->nd == 3 && s->n_inst == 1) return ST_LANE512;
+  return s->split_ok && (k != 0 || s->halo) ? ST_SPLIT : ST_LANE;
+}
+
 template <int ND, int PHYS, int FLUX, class R, int MODE, bool HANG, bool FUSE>
 void stage_t(h3c_solver s, const double* qin, double* out) {
+  const StageKernel kernel = stage_kernel(s);
   Launch L(s, MODE == 0 ? K_STAGE1 : K_STAGE2);
   if (PHYS == EULER && FLUX == AUSM && s->desc.reconstruction == H3C_RECON_MUSCL) {
     const bool two = ND == 2 && muscl_split(s);
@@ -423,7 +460,7 @@ void stage_t(h3c_solver s, const double* qin, double* out) {
                  s->pc, s->d_sc, &s->d_sc->dtmin_ord, s->needs_periodic ? s->d_gsrc : nullptr);
     return;
   }
-  if (PHYS == CNS && s->tile && s->halo && s->cns_ok) {
+  if (PHYS == CNS && kernel == ST_HALO) {
     int grid = s->persist_blocks > 0 ? s->persist_blocks : s->cns_bps * num_sms();
     grid = (int)std::max<long long>(1, std::min<long long>(grid, s->ntiles));
     const CnsHaloGeom ch{HaloGeom{s->d_lnb, s->d_hids, s->d_hoff, s->d_grp, s->d_goff, s->hmax}, s->d_h1end, s->d_hnb,
@@ -433,17 +470,17 @@ void stage_t(h3c_solver s, const double* qin, double* out) {
                    s->d_sc, &s->d_sc->dtmin_ord, &s->d_sc->status, grid, s->cns_smem, s->stream, s->d_gsl);
     return;
   }
-  if (PHYS == EULER && FLUX == AUSM && s->tile && s->euler_kernel == 3 && s->warp_bps > 0) {
+  if (PHYS == EULER && FLUX == AUSM && kernel == ST_WARP) {
     warp_stage(ND, std::is_same<R, float>::value, MODE, HANG, FUSE, qin, out, geometry(s), s->pc, s->d_sc,
                &s->d_sc->dtmin_ord, s->stream);
     return;
   }
-  if (PHYS == EULER && FLUX == AUSM && s->tile && (s->euler_kernel == 2 || s->euler_kernel == 3)) {  // per cell
+  if (PHYS == EULER && FLUX == AUSM && kernel == ST_CELL) {
     k_stage_ausm_cell<ND, R, MODE, HANG, FUSE><<<blocks(s->n_int), kBlock, 0, s->stream>>>(
         qin, out, geometry(s), s->pc, s->d_sc, &s->d_sc->dtmin_ord);
     return;
   }
-  if (PHYS == EULER && FLUX == AUSM && s->tile && s->halo && s->halo_ok && s->euler_kernel == 0) {
+  if (PHYS == EULER && FLUX == AUSM && kernel == ST_HALO) {
     int grid = s->persist_blocks > 0 ? s->persist_blocks : s->halo_bps * num_sms();
     grid = (int)std::max<long long>(1, std::min<long long>(grid, s->ntiles));
     HaloGeom hg{s->d_lnb, s->d_hids, s->d_hoff, s->d_grp, s->d_goff, s->hmax};
@@ -452,7 +489,7 @@ void stage_t(h3c_solver s, const double* qin, double* out) {
     return;
   }
   if constexpr (ND == 3) {
-    if (PHYS == EULER && FLUX == AUSM && s->tile && s->euler_kernel == 4 && s->n_inst == 1) {
+    if (PHYS == EULER && FLUX == AUSM && kernel == ST_LANE512) {
       // 512-cell tiles (8x8x8 Morton bricks), two blocks of 512 threads per SM
       constexpr int TB = 512;
       constexpr size_t smem = ausm_smem_bytes<R, ND, TB>();
@@ -470,7 +507,7 @@ void stage_t(h3c_solver s, const double* qin, double* out) {
       return;
     }
   }
-  if (PHYS == EULER && FLUX == AUSM && s->tile && s->split_ok) {
+  if (PHYS == EULER && FLUX == AUSM && kernel == ST_SPLIT) {
     const long long grid = s->persist_blocks > 0 ? std::min<long long>(s->persist_blocks, s->ntiles) : s->ntiles;
     const SplitGeom sg{(const uint4*)s->d_pack, (const uint2*)s->d_pack,
                        HaloGeom{s->d_lnb, s->d_hids, s->d_hoff, s->d_grp, s->d_goff, 0}};
@@ -478,8 +515,7 @@ void stage_t(h3c_solver s, const double* qin, double* out) {
                 &s->d_sc->dtmin_ord, (unsigned)std::max<long long>(1, grid), s->split_smem, s->stream);
     return;
   }
-  // tables beyond the slots' 15 or the cell ids' 29 bits: the per-lane tile kernel, which needs none
-  if (PHYS == EULER && FLUX == AUSM && s->tile) {
+  if (PHYS == EULER && FLUX == AUSM && kernel == ST_LANE) {
     constexpr size_t smem = ausm_smem_bytes<R, ND>();
     static bool attr = false;  // one opt-in per instantiation (dynamic smem above 48 KB)
     if (!attr) {
@@ -492,7 +528,7 @@ void stage_t(h3c_solver s, const double* qin, double* out) {
         qin, out, geometry(s), s->pc, s->d_sc, &s->d_sc->dtmin_ord);
     return;
   }
-  if (PHYS == EULER && s->tile) {
+  if (PHYS == EULER && kernel == ST_TILE) {
     constexpr size_t smem = tile_smem_bytes<R, ND>();
     static bool attr = false;  // one opt-in per instantiation (dynamic smem above 48 KB)
     if (!attr) {
@@ -504,11 +540,8 @@ void stage_t(h3c_solver s, const double* qin, double* out) {
         qin, out, geometry(s), s->pc, s->d_sc, &s->d_sc->dtmin_ord);
     return;
   }
-  // one grid without coarse/fine faces: two cells per thread (neighbour entries are cells then, never groups)
   if constexpr ((PHYS == HEAT || PHYS == ADVECTION) && !HANG) {
-    // from one full wave of k_stage's blocks on; below, a thread per cell finishes sooner (32,768 heat cells:
-    // 7.0 us against 8.5)
-    if (s->n_inst == 1 && s->n_int >= 6LL * kBlock * num_sms()) {
+    if (scalar_pairs(s)) {
       launch_chain(k_stage_scalar<ND, PHYS, FLUX, MODE, FUSE>, blocks((s->n_int + 1) / 2), kBlock, 0, s->stream, qin, out,
                    geometry(s), s->pc, s->d_sc, &s->d_sc->dtmin_ord);
       return;
@@ -1510,8 +1543,6 @@ int h3c_apply_bcs(h3c_solver s, int which) {
 
 // Solver::solve (solver.hpp:140-145): apply_bcs(lhs), set_dt, evolve, advance.
 // Per-stage preparation of a stage input q: CNS cell slopes or MUSCL gradients.
-static bool cns_tile_active(h3c_solver s) { return s->desc.physics == H3C_CNS && s->tile && s->halo && s->cns_ok; }
-
 static void prepare_stage(h3c_solver s, const double* q, int which) {
   if (s->desc.physics == H3C_CNS) {
     if (!cns_tile_active(s)) launch_slopes(s, which);  // the tile kernel computes slopes itself
@@ -2108,24 +2139,49 @@ int h3c_set_option(h3c_solver s, int option, int value) {
 int h3c_kernel_info(h3c_solver s, int64_t* info, int n) {
   if (!s || !info || n < 0) return H3C_E_INVALID;
   if (!s->has_grid) return s->fail(H3C_E_STATE, "h3c_kernel_info: no grid");
-  const bool euler = s->desc.physics == H3C_EULER && s->desc.reconstruction != H3C_RECON_MUSCL;
-  const bool cns = cns_tile_active(s);
-  const bool halo = cns || (euler && s->desc.flux == H3C_FLUX_AUSM && s->tile && s->halo && s->halo_ok);
-  const long long bps = cns ? s->cns_bps : s->halo_bps;
-  const int64_t grid = halo ? std::max<long long>(1, std::min<long long>(s->persist_blocks > 0 ? s->persist_blocks
-                                                                         : bps * num_sms(),
-                                                                         s->ntiles))
-                            : (s->persist_blocks > 0 ? std::min<long long>(s->persist_blocks, s->ntiles) : s->ntiles);
-  const bool ausm_tile = euler && s->desc.flux == H3C_FLUX_AUSM && s->tile;
-  const bool tile512 = ausm_tile && s->euler_kernel == 4 && s->nd == 3 && s->n_inst == 1;
-  const bool warpk = ausm_tile && s->euler_kernel == 3 && s->warp_bps > 0;
-  const bool cellk = ausm_tile && (s->euler_kernel == 2 || s->euler_kernel == 3) && !warpk;
-  const bool halo_used = halo && (cns || s->euler_kernel == 0);
-  const int64_t v[8] = {tile512 ? 5 : warpk ? 4 : cellk ? 3 : halo_used ? 2 : (euler && s->tile ? 1 : 0),
-                        (s->halo_ok || s->cns_ok) ? s->hmax : 0,
-                        s->halo_maxh, (int64_t)std::llround(1000.0 * s->halo_mean), bps, grid,
-                        (int64_t)(cns ? s->cns_smem : s->halo_smem), s->ntiles};
-  for (int i = 0; i < n && i < 8; ++i) info[i] = v[i];
+  const bool mixed = s->desc.precision == H3C_MIXED, d2 = s->nd == 2;
+  const StageKernel k = stage_kernel(s);
+  const bool cns = k == ST_HALO && s->desc.physics == H3C_CNS;
+  long long grid = blocks(s->n_int), tiles = s->ntiles, bps = 0, slots = 0;
+  size_t smem = 0;
+  switch (k) {
+    case ST_HALO:
+      bps = cns ? s->cns_bps : s->halo_bps;
+      slots = s->hmax;
+      smem = cns ? s->cns_smem : s->halo_smem;
+      break;
+    case ST_SPLIT:
+      slots = split_halo_slots(s->nd);
+      smem = s->split_smem;
+      break;
+    case ST_WARP:
+      smem = warp_smem_bytes(s->nd, mixed);
+      break;
+    case ST_LANE512:
+      smem = mixed ? ausm_smem_bytes<float, 3, 512>() : ausm_smem_bytes<double, 3, 512>();
+      tiles = (s->n_int + 511) / 512;
+      break;
+    case ST_LANE:
+      smem = d2 ? (mixed ? ausm_smem_bytes<float, 2>() : ausm_smem_bytes<double, 2>())
+                : (mixed ? ausm_smem_bytes<float, 3>() : ausm_smem_bytes<double, 3>());
+      break;
+    case ST_TILE:
+      smem = d2 ? (mixed ? tile_smem_bytes<float, 2>() : tile_smem_bytes<double, 2>())
+                : (mixed ? tile_smem_bytes<float, 3>() : tile_smem_bytes<double, 3>());
+      break;
+    case ST_PER_CELL:
+      if (s->desc.reconstruction == H3C_RECON_MUSCL && muscl_split(s)) grid = blocks(2 * s->n_int);
+      else if (scalar_pairs(s)) grid = blocks((s->n_int + 1) / 2);
+      break;
+    case ST_CELL: break;
+  }
+  if (k == ST_HALO) grid = s->persist_blocks > 0 ? s->persist_blocks : bps * num_sms();
+  else if (k == ST_SPLIT || k == ST_LANE || k == ST_LANE512) grid = s->persist_blocks > 0 ? s->persist_blocks : tiles;
+  if (k == ST_HALO || k == ST_SPLIT || k == ST_LANE || k == ST_LANE512)
+    grid = std::max<long long>(1, std::min<long long>(grid, tiles));
+  const int64_t v[9] = {k, slots, s->halo_maxh, (int64_t)std::llround(1000.0 * s->halo_mean), bps, grid,
+                        (int64_t)smem, s->ntiles, cns && s->d_blist};
+  for (int i = 0; i < n && i < 9; ++i) info[i] = v[i];
   return H3C_OK;
 }
 

@@ -433,6 +433,8 @@ void split_pack(int nd, const unsigned short* lnb, const unsigned char* lvl, lon
   k_split_pack<<<nb, kBlock, 0, st>>>(nd, lnb, lvl, ld, n, (uint4*)pack, (uint2*)pack);
 }
 
+int split_halo_slots(int nd) { return nd == 2 ? split_slots<2, double>() : split_slots<3, double>(); }
+
 size_t split_smem_bytes(int nd, bool mixed) {
   if (nd == 2) return mixed ? split_layout_bytes<2, float>() : split_layout_bytes<2, double>();
   return mixed ? split_layout_bytes<3, float>() : split_layout_bytes<3, double>();

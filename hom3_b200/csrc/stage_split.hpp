@@ -18,7 +18,8 @@ size_t split_pack_bytes(int nd, long long n);
 void split_pack(int nd, const unsigned short* lnb, const unsigned char* lvl, long long ld, long long n, void* pack,
                 cudaStream_t st);
 
-// Dynamic shared memory of one block.
+// Halo entries a block keeps in shared memory, and its dynamic shared memory.
+int split_halo_slots(int nd);
 size_t split_smem_bytes(int nd, bool mixed);
 // Opts the instantiations a solver launches (stage_modes, with or without
 // coarse/fine faces) into their dynamic shared memory where that needs an

@@ -309,7 +309,7 @@ int h3c_launches(h3c_solver s, int64_t* n);
  * H3C_OPT_GRAPHS       replay runs of steps from a captured CUDA graph (default 1)
  * H3C_OPT_HALO_KERNEL  the halo-staged tile kernels (each tile and its halo copied into shared
  *                      memory by bulk copies) may be used: the CNS stage and H3C_OPT_EULER_KERNEL 0
- *                      (default 1; 0: CNS steps in the per-cell kernel, Euler kernel 0 in the split one) */
+ *                      (default 1; 0: CNS steps in the per-cell kernel, Euler kernel 0 in the per-lane one) */
 #define H3C_OPT_TILE_KERNEL 1
 #define H3C_OPT_GRAPHS 2
 #define H3C_OPT_HALO_KERNEL 3
@@ -326,19 +326,20 @@ int h3c_launches(h3c_solver s, int64_t* n);
 #define H3C_OPT_HALO_SLOTS 6
 /* H3C_OPT_EULER_KERNEL  the Euler/AUSM stage kernel (with the tile kernels on): 0 the halo-staged
  *                       tile kernel when its tables exist, 1 (the default) the split tile kernel
- *                       (flux splits once per cell; grids beyond its tables' indices: the per-lane one),
+ *                       (flux splits once per cell; from 2^29 cells on the per-lane one),
  *                       2 one thread per cell, faces from both sides, 3 one warp per 32 Morton cells
  *                       (each face state once per warp, each face between two of its cells once),
  *                       4 the per-lane tile kernel on 512-cell tiles (8x8x8 Morton bricks, 512-thread
  *                       blocks; 3D single grids, otherwise kernel 1) */
 #define H3C_OPT_EULER_KERNEL 7
 int h3c_set_option(h3c_solver s, int option, int value);
-/* The Euler stage launch in use (no hom3 counterpart): info[0] kernel (0 per
- * cell, 1 split tile, 2 halo-staged tile, 3 the per-cell AUSM kernel, 4 the warp-tiled AUSM
- * kernel, 5 the per-lane tile kernel on 512-cell tiles), [1] halo slots per tile, [2]
- * largest tile halo, [3] mean tile halo x 1000, [4] resident blocks per SM
- * of the halo-staged kernel, [5] blocks launched, [6] its dynamic shared
- * memory in bytes, [7] 256-cell tiles; the first n entries are written. */
+/* The stage launch in use (no hom3 counterpart): info[0] kernel (0 per cell, 1 split tile,
+ * 2 halo-staged tile (Euler or CNS), 3 the per-cell AUSM kernel, 4 the warp-tiled AUSM kernel,
+ * 5 the per-lane tile kernel on 512-cell tiles, 6 on 256-cell tiles, 7 the LLF tile kernel), its
+ * [1] halo slots per tile (0: keeps none), [4] resident blocks per SM (halo-staged, else 0),
+ * [5] blocks launched, [6] dynamic shared memory in bytes, [8] 1 where the CNS kernel is the variant
+ * for brick grids; of the grid's tables [2] largest and [3] mean tile halo x 1000, [7] 256-cell
+ * tiles.  The first n entries are written. */
 int h3c_kernel_info(h3c_solver s, int64_t* info, int n);
 /* Self-test of the device reciprocal / reciprocal square root the kernels
  * use in place of division (n <= 2^24 positive inputs, host arrays). */
