@@ -77,6 +77,7 @@ SIGNATURES = {
     "h3c_state_device": (_i32, [_vp, _i32, _P(_P(_dbl)), _P(_i64)]),
     "h3c_device_order": (_i32, [_vp, _P(_i64)]),
     "h3c_get_stream": (_i32, [_vp, _P(_vp)]),
+    "h3c_wait_stream": (_i32, [_vp, _vp]),
     "h3c_sizes": (_i32, [_vp, _P(_i64), _P(_i64), _P(_i32)]),
     "h3c_solve": (_i32, [_vp, _i64]),
     "h3c_stages": (_i32, [_vp, _P(_i32)]),

@@ -164,6 +164,7 @@ struct h3c_solver_s {
   long long launches = 0;
   bool prof = false;
   std::vector<cudaEvent_t> ev_pool;
+  cudaEvent_t ev_wait = nullptr;  // h3c_wait_stream
   std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> prof_rec;
 
   int fail(int code, const char* fmt, ...) {
@@ -751,6 +752,7 @@ int h3c_destroy(h3c_solver s) {
   if (s->h_sc) cudaFreeHost(s->h_sc);
   for (auto& r : s->prof_rec) { cudaEventDestroy(r.second.first); cudaEventDestroy(r.second.second); }
   for (auto e : s->ev_pool) cudaEventDestroy(e);
+  if (s->ev_wait) cudaEventDestroy(s->ev_wait);
   if (s->stream && s->own_stream) cudaStreamDestroy(s->stream);
   delete s;
   return H3C_OK;
@@ -1511,6 +1513,26 @@ int h3c_device_order(h3c_solver s, int64_t* perm) {
 int h3c_get_stream(h3c_solver s, void** stream) {
   if (!s || !stream) return H3C_E_INVALID;
   *stream = (void*)s->stream;
+  return H3C_OK;
+}
+
+int h3c_wait_stream(h3c_solver s, void* stream) {
+  if (!s) return H3C_E_INVALID;
+  const cudaStream_t st = (cudaStream_t)stream;
+  if (st == s->stream) return H3C_OK;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(st, &cap);
+  if (e == cudaErrorStreamCaptureImplicit || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return H3C_OK;
+  }
+  if (e == cudaSuccess) e = cudaStreamQuery(st);
+  if (e == cudaSuccess) return H3C_OK;  // idle: nothing to wait for
+  if (e != cudaErrorNotReady) return s->cuda(e, "h3c_wait_stream");
+  cudaGetLastError();
+  if (!s->ev_wait) H3C_CUDA(s, cudaEventCreateWithFlags(&s->ev_wait, cudaEventDisableTiming));
+  H3C_CUDA(s, cudaEventRecord(s->ev_wait, st));
+  H3C_CUDA(s, cudaStreamWaitEvent(s->stream, s->ev_wait, 0));
   return H3C_OK;
 }
 

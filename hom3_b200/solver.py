@@ -219,14 +219,26 @@ class Solver:
         self.n_cells, self.first_ghost = n, int(first_ghost)
         self._grid = (g, nb, xc, ln, bc, arr)  # the tables h3c_write_vtk is handed again
 
+    def _handed_over(self, t):
+        """Address of a CUDA tensor for the library, whose next work waits for what torch's current stream still has
+        to do: the solver's stream is another one, and knows neither of the kernels that fill the tensor nor of those
+        that still use the memory the caching allocator gave it.  (Calls that take tensors return only when the
+        solver's stream is done, so what torch runs next finds them finished.)"""
+        import torch
+        dev = t.get_device()
+        if dev == torch.cuda.current_device():
+            self._check(lib().h3c_wait_stream(self.h, torch._C._cuda_getCurrentRawStream(dev)))
+        else:
+            torch.cuda.current_stream(dev).synchronize()
+        return C.cast(t.data_ptr(), C.POINTER(C.c_double))
+
     def set_state(self, q, which=LHS):
         """q: [nv][n_cells] float64, a numpy array or a CUDA tensor (copied device to device)."""
         if hasattr(q, "is_cuda") and q.is_cuda:
             import torch
             t = q.contiguous()
             assert t.dtype == torch.float64 and tuple(t.shape) == (self.nv, self.n_cells), (t.dtype, t.shape)
-            self._check(lib().h3c_set_state(self.h, which, C.cast(t.data_ptr(), C.POINTER(C.c_double)),
-                                            self.n_cells))
+            self._check(lib().h3c_set_state(self.h, which, self._handed_over(t), self.n_cells))
             return
         q = np.ascontiguousarray(q, np.float64)
         assert q.shape == (self.nv, self.n_cells), q.shape
@@ -255,8 +267,7 @@ class Solver:
         if out is not None and hasattr(out, "is_cuda") and out.is_cuda:
             import torch
             assert out.dtype == torch.float64 and tuple(out.shape) == (self.nv, self.n_cells) and out.is_contiguous()
-            self._check(lib().h3c_get_state(self.h, which, C.cast(out.data_ptr(), C.POINTER(C.c_double)),
-                                            self.n_cells))
+            self._check(lib().h3c_get_state(self.h, which, self._handed_over(out), self.n_cells))
             return out
         if out is None:
             out = np.empty((self.nv, self.n_cells), np.float64)
@@ -383,8 +394,7 @@ class Solver:
             lam = dJ_dqN.contiguous()
             assert lam.dtype == torch.float64 and tuple(lam.shape) == (self.nv, self.n_cells)
             grad = torch.empty_like(lam) if out is None else out
-            self._check(lib().h3c_adjoint(self.h, nsteps, every, C.cast(lam.data_ptr(), C.POINTER(C.c_double)),
-                                          C.cast(grad.data_ptr(), C.POINTER(C.c_double)), _dp(dts)))
+            self._check(lib().h3c_adjoint(self.h, nsteps, every, self._handed_over(lam), self._handed_over(grad), _dp(dts)))
             return grad, dts
         lam = np.ascontiguousarray(dJ_dqN, np.float64)
         assert lam.shape == (self.nv, self.n_cells)

@@ -233,6 +233,11 @@ int h3c_set_velocity(h3c_solver s, const double* u, int64_t ld);
 int h3c_state_device(h3c_solver s, int which, double** ptr, int64_t* ld);
 int h3c_device_order(h3c_solver s, int64_t* perm);
 int h3c_get_stream(h3c_solver s, void** stream);
+/* The solver's next work waits for all that is enqueued on `stream` (a cudaStream_t of the solver's
+ * device; NULL: the default stream) so far: before device memory that another stream writes or still
+ * uses is handed to a call.  The solver's own stream is a non-blocking one.  No wait for a stream
+ * under capture, which runs nothing. */
+int h3c_wait_stream(h3c_solver s, void* stream);
 int h3c_sizes(h3c_solver s, int64_t* n_cells, int64_t* first_ghost, int* nv);
 
 /* ---- stepping: Solver::solve (solver.hpp:140-145), n times.  The step runs
