@@ -1144,14 +1144,10 @@ static int set_grids(h3c_solver s, int ninst, const h3c_grid* grids) {
     s->warp_bps = warp_prepare(nd, s->desc.precision == H3C_MIXED);
   if (cns_tables) {
     const bool mixed = s->desc.precision == H3C_MIXED;
-    // the brick variant where every tile is one; a grid of a few tiles may fit only the general one
-    size_t smem = 0;
-    int bps = 0;
-    for (int brick = CH.brick ? 1 : 0; brick >= 0 && bps == 0; --brick) {
-      CH.brick = brick != 0;
-      smem = cns_halo_smem_bytes(nd, mixed, CH.base.hmax, CH.h1max, CH.brick);
-      bps = smem <= 227 * 1024 ? cns_halo_prepare(nd, mixed, stage_modes(s->desc.time_integration), smem, CH.brick) : 0;
-    }
+    // (the brick variant's layout stays below 160 KB whatever the second layer's size)
+    const size_t smem = cns_halo_smem_bytes(nd, mixed, CH.base.hmax, CH.h1max, CH.brick);
+    const int bps = smem <= 227 * 1024
+                        ? cns_halo_prepare(nd, mixed, stage_modes(s->desc.time_integration), smem, CH.brick) : 0;
     if (bps > 0 && CH.brick) {
       H3C_CUDA(s, cudaMalloc(&s->d_blist, sizeof(unsigned) * CH.blist.size()));
       H3C_CUDA(s, cudaMalloc(&s->d_bsel, sizeof(unsigned) * CH.bsel.size()));
