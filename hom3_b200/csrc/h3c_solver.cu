@@ -393,10 +393,12 @@ void launch_slopes_ptr(h3c_solver s, const double* q) {
 
 void launch_slopes(h3c_solver s, int which) { launch_slopes_ptr(s, s->d_q[which]); }
 
-// Two threads per cell in the 2D MUSCL kernels (muscl_kernels.cuh) up to one
-// block of them per SM.  SSP-RK3, 30 steps, us with one / two threads: 64^2
-// 1145 / 911, 128^2 1164 / 976, 256^2 1431 / 1684, 400^2 2809 / 2969.
-bool muscl_split(h3c_solver s) { return s->nd == 2 && s->n_int <= (long long)kBlock / 2 * num_sms(); }
+// Two threads per cell in the 2D MUSCL kernels (muscl_kernels.cuh) on grids of
+// less than two blocks of them per SM.  SSP-RK3, us per step with one / two
+// threads: 64^2 28.2 / 22.7, 128^2 28.9 / 24.9, 160^2 33.6 / 28.5, 192^2 34.4 /
+// 29.3; even from there (200^2 38.7 / 38.4, 256 x 148 29.8 / 30.8), 240^2 41.2 /
+// 45.9, 256^2 37.2 / 43.6.
+bool muscl_split(h3c_solver s) { return s->nd == 2 && s->n_int < (long long)kBlock * num_sms(); }
 
 // EXTENSION: limited least-squares gradients of the stage input (MUSCL)
 // ghosts_too: the periodic ghosts' copies as well (the adjoint reads them; the stage reads through d_gsrc)
@@ -415,8 +417,9 @@ void launch_grad(h3c_solver s, const double* q, bool ghosts_too) {
 }
 
 // Two cells per thread in the stages of heat and advection (k_stage_scalar): one grid without coarse/fine faces
-// (neighbour entries are cells then, never groups), from one full wave of k_stage's blocks on; below, a thread per
-// cell finishes sooner (32,768 heat cells: 7.0 us against 8.5).
+// (neighbour entries are cells then, never groups), from one full wave of k_stage's blocks on (227,328 cells).  Us
+// per step, a thread per cell / per pair: heat 216,000 cells 4.7 / 6.2, 230,702 6.0 / 5.95, 262,144 6.4 / 6.2,
+// 512,000 8.7 / 8.6; advection 193,600 6.2 / 6.3, 228,000 6.2 / 6.0, 262,144 7.3 / 7.0.
 bool scalar_pairs(h3c_solver s) {
   return (s->desc.physics == H3C_HEAT || s->desc.physics == H3C_ADVECTION) && s->nsub == 0 && s->n_inst == 1 &&
          s->n_int >= 6LL * kBlock * num_sms();

@@ -91,8 +91,9 @@ template <int SPLIT> __device__ __forceinline__ long long split_cell(int& sub) {
 
 // SPLIT 2 (2D): two threads per cell, each with half of the variables.  Small
 // grids have too few cells to hide a thread's chain of a thousand dependent
-// instructions: 256^2 cells are 3.5 warps per scheduler, of which the FP64
-// pipe sees a third.
+// instructions: 64^2 cells are a fifth of a warp per scheduler, 128^2 not
+// quite one.  Up to less than two blocks of the split kernels per SM they gain
+// (muscl_split, h3c_solver.cu).
 template <int ND, bool HANG, int SPLIT>
 __global__ void __launch_bounds__(kBlock) k_muscl_grad(const double* q, const double* __restrict__ xc,
                                                        Geometry g, PhysConst pc, double limiter_k,
