@@ -40,6 +40,16 @@ def log(*a):
     print(*a, file=sys.stderr, flush=True)
 
 
+def stage2_traffic(kernel, precision, n_cells):
+    """DRAM bytes of one second RK2 stage of n_cells tree cells by the stage kernel in use, as ncu counted them per
+    cell on the default tree; None for a kernel and precision that were not captured."""
+    try:
+        with open(os.path.join(ROOT, "profiles", "stage2_traffic.json")) as f:
+            return json.load(f)["kernels"][kernel][precision]["dram_bytes_per_leaf_cell"] * n_cells
+    except (OSError, ValueError, KeyError):
+        return None
+
+
 def peaks():
     p = os.path.join(ROOT, "MEASURED_PEAKS.json")
     try:
@@ -1277,21 +1287,15 @@ def main():
     bytes_st1 = fg * (2 * 5 * 8 + 6 * 4 + 1)
     st2_avg = st2_ms / max(st2_n, 1)
     achieved = bytes_st2 / (st2_avg * 1e-3) / 1e9 if st2_n else None
-    traffic = None
-    tp = os.path.join(ROOT, "profiles", "stage2_traffic.json")
-    if os.path.exists(tp):
-        try:
-            d = json.load(open(tp))
-            traffic = d["dram_bytes_per_leaf_cell"] * fg
-        except Exception:
-            traffic = None
+    stage_kernel = s.kernel_info()
+    traffic = stage2_traffic(stage_kernel["kernel"], args.precision, fg)
     step_bytes = bytes_st1 + bytes_st2
     line = {
         "metric": "cell-updates/s", "value": value, "unit": "cell-updates/s", "n_gpus": ws, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_max / args.steps, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f64" if args.precision == "fp64" else "f32-flux/f64-state",
         "data": "synthetic", "config": workload_config(args, t),
-        "roofline": {"bound": "hbm", "kernel": "k_stage (second RK stage)", "achieved": achieved, "peak": peak,
+        "roofline": {"bound": "hbm", "kernel": stage_kernel["kernel"] + " (second RK stage)", "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": (achieved / peak) if achieved else None, "traffic": traffic,
                      "peak_source": peak_kind, "algorithmic_bytes_per_launch": bytes_st2,
                      "avg_launch_ms": st2_avg,
@@ -1312,7 +1316,7 @@ def main():
     if adj is not None:
         line["adjoint"] = adj
     line["grid_build"] = getattr(args, "grid_build", None)
-    line["stage_kernel"] = s.kernel_info()
+    line["stage_kernel"] = stage_kernel
     line["autotune"] = tune
     r64, r32 = hb_fma_rates()
     line["fma_rates"] = {"fp64_tflops": 2 * r64 / 1e12, "fp32_tflops": 2 * r32 / 1e12,
