@@ -207,7 +207,7 @@ __device__ __forceinline__ void flag_timeout(const Scalars* sc, int* status) {
 // every kernel before it has finished and its writes are visible.  The steps of
 // small grids are chains of kernels of a few microseconds, whose launch gaps
 // this hides (with the scalar work moved into the conditions' kernel, see
-// StepBegin: 256^2 MUSCL, SSP-RK3, 30 steps 2187 -> 1465 us; 48 coupled
+// StepBegin: 256^2 MUSCL, SSP-RK3, 30 steps 2187 -> 1353 us; 48 coupled
 // 512 x 192 steps 2458 -> 1481 us).  Every kernel launched that way starts
 // with this call.
 // The set-up tables do not change while kernels run, so what a block needs of
@@ -1145,7 +1145,7 @@ __global__ void __launch_bounds__(kBlock) k_stage(const double* qin, double* out
 // dt / length is divided once per level and block.  2048^2 advection, LLF,
 // forward Euler: 73.8 us per stage in k_stage -> 59.4 here; 100^3 heat: 16.9
 // -> 14.8 (with the events' overhead of about 5).  What is left is latency:
-// 3.4 TB/s of DRAM traffic, issue slots and L1 under half used.  Prefetching
+// 3.3 TB/s of DRAM traffic, issue slots and L1 half used.  Prefetching
 // the tables of a block one wave ahead into L2 gained 3% in advection and
 // lost 8% in heat; left out.
 // ---------------------------------------------------------------------------

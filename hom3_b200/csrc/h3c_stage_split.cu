@@ -16,14 +16,14 @@
 // face once and handed the flux over, which took two more barriers and 30 KB
 // of flux rows, and its border cells -- a third of an 8x8x4 brick's faces --
 // recomputed the neighbour's primitive state in divergent branches (20.7 of
-// 32 lanes active; 28.7 here).  1,448,336-cell 3D tree, RK2, microseconds per
+// 32 lanes active; 27.5-28.5 here).  1,448,336-cell 3D tree, RK2, microseconds per
 // stage with the events' overhead (about 4), same GPU: FP64 98.6 / 111.2
 // before, 84.1 / 105.0 here; FP32 fluxes 86.3 / 101.5 before, 70.0 / 82.1
 // here; 24 2D grids of 2.3 M cells, FP32 fluxes: 85.0 / 99.1 before,
 // 67.9 / 80.3 here.
 //
-// What bounds it: the shared-memory pipe in FP64 (60-70% of its cycles by
-// ncu), and in both the latency of the gathers ahead of the one barrier at
+// What bounds it: the pipe of shared memory and L1 in FP64 (59-63% of its
+// peak by ncu), and in both the latency of the gathers ahead of the one barrier at
 // 24-32 warps per SM.  At four blocks shared memory takes nearly the whole
 // L1, so a register spilled on the common path costs an L2 round trip.  Hence
 // the FP64 halo states land in shared memory by 8-byte asynchronous copies
