@@ -296,7 +296,11 @@ __global__ void __launch_bounds__(kHaloTile, H3C_CNS_MINB)
     const bool ok = mbar_wait_bounded(bar, (unsigned)(it & 1));
     cp_async_wait_all();
     if (!__syncthreads_and(ok)) {
-      if (tid == 0) flag_timeout(sc, status);
+      if (tid == 0) {
+        flag_timeout(sc, status);
+        // the block keeps its shared memory while its copies may still land there, for a second bounded wait
+        mbar_wait_bounded(bar, (unsigned)(it & 1));
+      }
       return;
     }
 
